@@ -458,6 +458,11 @@ int build_ibm_lists3(efvm_ctx* c) {
     c->markers3_dev = nullptr;
     CUDA_TRY(c, cudaMalloc(&c->ghosts3_dev, std::max<size_t>(ghosts.size(), 1) * sizeof(IbmGhost3Dev)));
     CUDA_TRY(c, cudaMalloc(&c->markers3_dev, std::max<size_t>(markers.size(), 1) * sizeof(Marker3Dev)));
+    cudaFree(c->force_partials);
+    c->force_partials = nullptr;
+    c->ibm_desc.partials = nullptr;
+    const size_t nblocks = std::max(1, ibm3_force_blocks((int)markers.size(), (int)ghosts.size()));
+    CUDA_TRY(c, cudaMalloc(&c->force_partials, nblocks * 6 * sizeof(double)));
     if (!ghosts.empty())
         CUDA_TRY(c, cudaMemcpyAsync(c->ghosts3_dev, ghosts.data(), ghosts.size() * sizeof(IbmGhost3Dev),
                                     cudaMemcpyHostToDevice, S(c)));
@@ -473,6 +478,8 @@ int build_ibm_lists3(efvm_ctx* c) {
     d.markers3 = c->markers3_dev;
     d.sample_offset = offset;
     d.force_out = c->force_out;
+    d.partials = c->force_partials;
+    d.counter = c->force_counter;
     return EFVM_OK;
 }
 
@@ -562,7 +569,13 @@ void enqueue_stage_kernel(efvm_ctx* c, int stage, double* uin, double* uout, boo
 // the bodies, the force history's control), first runs them here if a step
 // left them pending: the kernel does nothing otherwise.
 static int finish_forces(efvm_ctx* c) {
-    if (!c->ibm || is_3d(c)) return EFVM_OK;
+    if (!c->ibm) return EFVM_OK;
+    if (is_3d(c)) {
+        // before the first geometry no step has run and there are no lists yet
+        if (c->ibm_desc.partials)
+            c->launches += launch_ibm3(c->g, c->ph, c->ibm_desc, c->U[0], c->st, true, false, 0, false, S(c), 1);
+        return EFVM_OK;
+    }
     c->launches += launch_ibm(c->g, c->ph, c->ibm_desc, c->U[0], c->st, 2, -1, 0, false, S(c), 1);
     return EFVM_OK;
 }
@@ -570,11 +583,10 @@ static int finish_forces(efvm_ctx* c) {
 // Launch the kernels of one substage at RK stage `stage` (0..2, or 3 = Euler):
 // [step set-up +] IBM mirror of uin, the stage, the IBM forces of uout.
 void enqueue_substage(efvm_ctx* c, int stage, double* uin, double* uout, bool with_setup) {
-    if (c->ibm && is_3d(c)) {  // spheres: [set-up], mirror, stage, forces, all on the main stream
-        if (with_setup) c->launches += launch_step_setup(c->ph, c->st, true, S(c));
-        c->launches += launch_mirror3(c->g, c->ph, c->ibm_desc, uin, true, S(c));
+    if (c->ibm && is_3d(c)) {  // spheres: [set-up and] mirror, stage, forces, all on the main stream
+        c->launches += launch_ibm3(c->g, c->ph, c->ibm_desc, uin, c->st, false, true, with_setup, true, S(c));
         enqueue_stage_kernel(c, stage, uin, uout);
-        c->launches += launch_forces3(c->g, c->ph, c->ibm_desc, uout, c->st, true, S(c));
+        c->launches += launch_ibm3(c->g, c->ph, c->ibm_desc, uout, c->st, true, false, 0, true, S(c));
         return;
     }
     if (c->ibm) c->launches += launch_ibm(c->g, c->ph, c->ibm_desc, uin, c->st, -1, stage, with_setup, true, S(c));
@@ -594,21 +606,23 @@ void enqueue_substage(efvm_ctx* c, int stage, double* uin, double* uout, bool wi
 // step saves into the other parity's buffer.
 int enqueue_rk3_step(efvm_ctx* c) {
     double* bufs[4] = {c->U[0], c->U[1], c->U[2], c->U[0]};
-    if (c->ibm && is_3d(c)) {
-        for (int s = 0; s < 3; ++s) enqueue_substage(c, s, bufs[s], bufs[s + 1], s == 0);
-        return EFVM_OK;
-    }
+    auto ibm = [&](double* q, int force_stage, int mirror_stage, int setup, bool pdl, cudaStream_t s, int deferred) {
+        if (is_3d(c))
+            return launch_ibm3(c->g, c->ph, c->ibm_desc, q, c->st, force_stage >= 0, mirror_stage >= 0, setup, pdl, s,
+                               deferred);
+        return launch_ibm(c->g, c->ph, c->ibm_desc, q, c->st, force_stage, mirror_stage, setup, pdl, s, deferred);
+    };
     // the first launch: the forces of the previous step's last stage (when pending),
     // the set-up and the mirror of stage 1; bufs[0] is both their state and its input
-    if (c->ibm) c->launches += launch_ibm(c->g, c->ph, c->ibm_desc, bufs[0], c->st, 2, 0, 1, true, S(c), 1);
+    if (c->ibm) c->launches += ibm(bufs[0], 2, 0, 1, true, S(c), 1);
     else c->launches += launch_step_setup(c->ph, c->st, true, S(c));
     for (int s = 0; s < 3; ++s) {
         enqueue_stage_kernel(c, s, bufs[s], bufs[s + 1], true, c->ibm && s == 2);
         if (c->ibm && s < 2) {
             CUDA_TRY(c, cudaEventRecord(c->ev_fork[s], S(c)));
             CUDA_TRY(c, cudaStreamWaitEvent(c->side, c->ev_fork[s], 0));
-            c->launches += launch_ibm(c->g, c->ph, c->ibm_desc, bufs[s + 1], c->st, s, -1, 0, false, c->side);
-            c->launches += launch_ibm(c->g, c->ph, c->ibm_desc, bufs[s + 1], c->st, -1, s + 1, 0, true, S(c));
+            c->launches += ibm(bufs[s + 1], s, -1, 0, false, c->side, 0);
+            c->launches += ibm(bufs[s + 1], -1, s + 1, 0, true, S(c), 0);
         }
     }
     if (c->ibm) {
@@ -623,7 +637,7 @@ int capture_step_graph(efvm_ctx* c) {
         cudaGraphExecDestroy(c->graph_exec);
         c->graph_exec = nullptr;
     }
-    if (c->ibm && !is_3d(c) && !c->side) {
+    if (c->ibm && !c->side) {
         CUDA_TRY(c, cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking));
         for (auto& ev : c->ev_fork) CUDA_TRY(c, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
         CUDA_TRY(c, cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming));
@@ -1009,6 +1023,10 @@ int efvm_download_state(efvm_ctx* c, double* base, int64_t si, int64_t sj, int64
 static int transfer_state3(efvm_ctx* c, double* base, int64_t si, int64_t sj, int64_t sk, int64_t sv, bool upload) {
     if (!c || !base) return fail(c, EFVM_ERR_INVALID_ARG, "null argument");
     if (!is_3d(c)) return transfer_state(c, base, si, sj, sv, upload);
+    if (upload) {  // pending forces read the state this replaces
+        const int rcf = finish_forces(c);
+        if (rcf) return rcf;
+    }
     const Geometry& g = c->g;
     int64_t lo = 0, hi = 0;
     const int64_t corners[4] = {(int64_t)(g.nx - 1) * si, (int64_t)(g.ny - 1) * sj, (int64_t)(g.nz - 1) * sk, 4 * sv};
@@ -1551,6 +1569,10 @@ int efvm_set_spheres(efvm_ctx* c, const efvm_sphere* sph, int32_t n, int32_t n_m
     if (!is_3d(c))
         return fail(c, EFVM_ERR_UNSUPPORTED,
                     "spheres are 3-D bodies: efvm_set_spheres needs nz > 1 (efvm_set_cylinders is the 2-D form)");
+    {  // pending forces belong to the bodies being replaced
+        const int rcf = finish_forces(c);
+        if (rcf) return rcf;
+    }
     if (n == 0) {
         c->ibm = false;
         c->graph_valid = false;
@@ -1698,13 +1720,13 @@ int efvm_profile_steps(efvm_ctx* c, int64_t n_steps, double out_ms[4]) {
         float ms_stage = 0.f, ms_ibm = 0.f;
         for (int s = 0; s < 3; ++s) {
             if (c->ibm)
-                c->launches += is_3d(c) ? launch_mirror3(c->g, c->ph, ib, bufs[s], false, S(c))
+                c->launches += is_3d(c) ? launch_ibm3(c->g, c->ph, ib, bufs[s], c->st, false, true, 0, false, S(c))
                                         : launch_ibm(c->g, c->ph, ib, bufs[s], c->st, -1, s, 0, false, S(c));
             CUDA_TRY(c, cudaEventRecord(ev[2], S(c)));
             enqueue_stage_kernel(c, s, bufs[s], bufs[s + 1], false);
             CUDA_TRY(c, cudaEventRecord(ev[3], S(c)));
             if (c->ibm)
-                c->launches += is_3d(c) ? launch_forces3(c->g, c->ph, ib, bufs[s + 1], c->st, false, S(c))
+                c->launches += is_3d(c) ? launch_ibm3(c->g, c->ph, ib, bufs[s + 1], c->st, true, false, 0, false, S(c))
                                         : launch_ibm(c->g, c->ph, ib, bufs[s + 1], c->st, s, -1, 0, false, S(c));
             CUDA_TRY(c, cudaEventRecord(ev[4], S(c)));
             CUDA_TRY(c, cudaEventSynchronize(ev[4]));

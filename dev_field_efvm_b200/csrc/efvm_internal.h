@@ -323,14 +323,17 @@ int launch_ibm(const Geometry& g, const Physics& ph, const Ibm& ibm, double* q, 
 int launch_pack(const Geometry& g, const double* host_like, int64_t si, int64_t sj, int64_t sv, double* q,
                  int to_device, void* stream);
 // 3-D spheres: the solid mask with the stagnant/ambient re-seed of flipped
-// cells (spheres: n x 10 doubles as efvm_sphere), the ghost mirror of q before
-// a stage, and the marker and staircase forces of q after one (one block,
-// fixed-order sums, the marker force appended to the history when it is set).
+// cells (spheres: n x 10 doubles as efvm_sphere), and one launch of the IBM work
+// between stage kernels: the marker and staircase forces of q after a stage
+// (fixed-order sums, the marker force appended to the history when it is set;
+// deferred as in launch_ibm) and the ghost mirror of q before one, with `setup`
+// also the per-step set-up.
 int launch_geometry3(const Geometry& g, const Physics& ph, const double* spheres, int n, const double* stagnant,
                      const double* ambient, double* q, uint8_t* mask, void* stream);
-int launch_mirror3(const Geometry& g, const Physics& ph, const Ibm& ib, double* q, bool pdl, void* stream);
-int launch_forces3(const Geometry& g, const Physics& ph, const Ibm& ib, const double* q, DevState* st, bool pdl,
-                   void* stream);
+int launch_ibm3(const Geometry& g, const Physics& ph, const Ibm& ib, double* q, DevState* st, bool forces, bool mirror,
+                int setup, bool pdl, void* stream, int deferred = 0);
+// Force blocks of one launch (Ibm::partials holds 6 doubles of each).
+int ibm3_force_blocks(int n_markers, int n_ghost);
 // The same for a 3-D state: element (i, j, k, v) at i si + j sj + k sk + v sv.
 int launch_pack3(const Geometry& g, double* host_like, int64_t si, int64_t sj, int64_t sk, int64_t sv, double* q,
                  int to_device, void* stream);

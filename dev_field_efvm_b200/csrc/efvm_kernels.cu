@@ -2119,15 +2119,18 @@ int launch_geometry3(const Geometry& g, const Physics& ph, const double* spheres
     return 1;
 }
 
-int launch_mirror3(const Geometry& g, const Physics& ph, const Ibm& ib, double* q, bool pdl, void* stream) {
-    const int nb = ib.n_ghost > 0 ? (ib.n_ghost + 127) / 128 : 1;
-    launch_k(mirror3_kernel, dim3(nb), dim3(128), (cudaStream_t)stream, pdl, g, ph, ib, q);
-    return 1;
+int ibm3_force_blocks(int n_markers, int n_ghost) {
+    return (n_markers + IBM_THREADS - 1) / IBM_THREADS + (n_ghost + IBM_THREADS - 1) / IBM_THREADS;
 }
 
-int launch_forces3(const Geometry& g, const Physics& ph, const Ibm& ib, const double* q, DevState* st, bool pdl,
-                   void* stream) {
-    launch_k(forces3_kernel, dim3(1), dim3(FORCE3_THREADS), (cudaStream_t)stream, pdl, g, ph, ib, q, st);
+int launch_ibm3(const Geometry& g, const Physics& ph, const Ibm& ib, double* q, DevState* st, bool forces, bool mirror,
+                int setup, bool pdl, void* stream, int deferred) {
+    const int nfm = forces ? (ib.n_markers + IBM_THREADS - 1) / IBM_THREADS : 0;
+    const int nf = forces ? std::max(1, ibm3_force_blocks(ib.n_markers, ib.n_ghost)) : 0;
+    const int nm = mirror ? std::max(1, (ib.n_ghost + IBM_THREADS - 1) / IBM_THREADS) : 0;
+    if (nf + nm == 0) return 0;
+    launch_k(ibm3_kernel, dim3(nf + nm), dim3(IBM_THREADS), (cudaStream_t)stream, pdl, g, ph, ib, q, st, nfm, nf, setup,
+             deferred);
     return 1;
 }
 

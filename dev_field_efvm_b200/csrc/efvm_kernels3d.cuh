@@ -231,6 +231,7 @@ __global__ void __launch_bounds__(32 * WPB3, MINB3) stage3_kernel(StageArgs a, i
             st->completed = 1;
             st->step += 1;
             st->time += st->dt;
+            if (a.defer_forces) st->forces_pending = 1;
         } else {
             st->rk_stage = a.stage + 1;
             st->completed = 0;
@@ -654,39 +655,39 @@ __global__ void geometry3_kernel(Geometry g, Physics ph, const double* __restric
 // sample_trilinear, crates/cfd_ibm/src/lib.rs:106-149: primitive (rho, u, v, w,
 // p, T) at a located point from the fluid corners of its 2x2x2 block (clear
 // corner bits are solid), skipping non-positive or non-finite densities, the
-// weights renormalised; false when they sum below 1e-12.
+// weights renormalised; false when they sum below 1e-12.  The eight corner
+// states are loaded before any of them is used (every corner of a located block
+// is in bounds), so a sample waits for memory once and not eight times.
 __device__ __forceinline__ bool sample_trilinear3(const Geometry& g, const Physics& ph, const double* q,
                                                   unsigned fluid, const int lo[3], const double t[3], double out[6]) {
     const double gm1 = ph.gamma - 1.0;
+    U5 cu[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+        cu[c] = load5(q, g.plane, cidx3(g, lo[0] + (c >> 2), lo[1] + ((c >> 1) & 1), lo[2] + (c & 1)));
     double acc[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
     double total = 0.0;
 #pragma unroll
-    for (int di = 0; di < 2; ++di) {
-        const double wx = di == 0 ? 1.0 - t[0] : t[0];
-#pragma unroll
-        for (int dj = 0; dj < 2; ++dj) {
-            const double wy = dj == 0 ? 1.0 - t[1] : t[1];
-#pragma unroll
-            for (int dk = 0; dk < 2; ++dk) {
-                const double wz = dk == 0 ? 1.0 - t[2] : t[2];
-                if (!(fluid & (1u << (FLUID3_CORNER_SHIFT + 4 * di + 2 * dj + dk)))) continue;
-                const U5 u = load5(q, g.plane, cidx3(g, lo[0] + di, lo[1] + dj, lo[2] + dk));
-                if (!isfinite(u.r) || u.r <= 0.0) continue;
-                const double w = wx * wy * wz;
-                const double inv = 1.0 / u.r;
-                const double vu = u.mx * inv, vv = u.my * inv, vw = u.mz * inv;
-                const double ke = 0.5 * u.r * (vu * vu + vv * vv + vw * vw);
-                const double p = gm1 * (u.E - ke);
-                const double tt = p * inv / ph.r_gas;
-                acc[0] += w * u.r;
-                acc[1] += w * vu;
-                acc[2] += w * vv;
-                acc[3] += w * vw;
-                acc[4] += w * p;
-                acc[5] += w * tt;
-                total += w;
-            }
-        }
+    for (int c = 0; c < 8; ++c) {  // (di, dj, dk) = (c >> 2, (c >> 1) & 1, c & 1)
+        const double wx = (c >> 2) == 0 ? 1.0 - t[0] : t[0];
+        const double wy = ((c >> 1) & 1) == 0 ? 1.0 - t[1] : t[1];
+        const double wz = (c & 1) == 0 ? 1.0 - t[2] : t[2];
+        const U5 u = cu[c];
+        if (!(fluid & (1u << (FLUID3_CORNER_SHIFT + c)))) continue;
+        if (!isfinite(u.r) || u.r <= 0.0) continue;
+        const double w = wx * wy * wz;
+        const double inv = 1.0 / u.r;
+        const double vu = u.mx * inv, vv = u.my * inv, vw = u.mz * inv;
+        const double ke = 0.5 * u.r * (vu * vu + vv * vv + vw * vw);
+        const double p = gm1 * (u.E - ke);
+        const double tt = p * inv * ph.inv_r_gas;
+        acc[0] += w * u.r;
+        acc[1] += w * vu;
+        acc[2] += w * vv;
+        acc[3] += w * vw;
+        acc[4] += w * p;
+        acc[5] += w * tt;
+        total += w;
     }
     if (total < 1e-12) return false;
     const double inv = 1.0 / total;
@@ -699,10 +700,7 @@ __device__ __forceinline__ bool sample_trilinear3(const Geometry& g, const Physi
 // image point's density, pressure and temperature and the velocity mirrored
 // about the wall velocity, 2 u_w - u_image; a ghost whose sample fails keeps its
 // value.
-__global__ void mirror3_kernel(Geometry g, Physics ph, Ibm ib, double* q) {
-    pdl_wait_then_release();
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= ib.n_ghost) return;
+__device__ __forceinline__ void mirror_ghost3(const Geometry& g, const Physics& ph, const Ibm& ib, double* q, int t) {
     const IbmGhost3Dev gh = ib.ghosts3[t];
     if (!gh.valid) return;
     double im[6];
@@ -713,72 +711,135 @@ __global__ void mirror3_kernel(Geometry g, Physics ph, Ibm ib, double* q) {
     store5(q, g.plane, cidx3(g, gh.i, gh.j, gh.k), c);
 }
 
-// marker_force_system + compute_marker_loadings (crates/cfd_ibm/src/lib.rs:442-480,
-// 601-615) and wall_force_system (:309-395) over the state after a stage: one
-// block, each thread summing a strided share of the markers and of the solid
-// cells with fluid neighbours (the ghost list), then a fixed-order tree sum.
-constexpr int FORCE3_THREADS = 256;
-__global__ void __launch_bounds__(FORCE3_THREADS) forces3_kernel(Geometry g, Physics ph, Ibm ib, const double* q,
-                                                                  DevState* st) {
-    pdl_wait_then_release();
-    __shared__ double red[12][FORCE3_THREADS];
-    double f[12] = {0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0, 0};  // marker p, v; wall p, v
+// One marker's pressure and viscous force (marker_force_system +
+// compute_marker_loadings, crates/cfd_ibm/src/lib.rs:442-480,601-615).
+__device__ __forceinline__ void marker_load3(const Geometry& g, const Physics& ph, const Ibm& ib, const double* q,
+                                             int m, double f[6]) {
+    const Marker3Dev mk = ib.markers3[m];
+    if (!mk.valid) return;
+    double img[6];
+    if (!sample_trilinear3(g, ph, q, mk.fluid, mk.lo, mk.t, img)) return;
+    if (!(isfinite(img[4]) && isfinite(img[5]) && isfinite(img[1]) && isfinite(img[2]) && isfinite(img[3]))) return;
+    const double us[3] = {img[1] - mk.uw[0], img[2] - mk.uw[1], img[3] - mk.uw[2]};
+    const double udotn = us[0] * mk.normal[0] + us[1] * mk.normal[1] + us[2] * mk.normal[2];
+    const double mu = viscosity(ph, img[5]);
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+        const double ut = us[d] - udotn * mk.normal[d];
+        f[d] = -img[4] * mk.normal[d] * mk.area;
+        f[3 + d] = mu * ut / ib.sample_offset * mk.area;
+    }
+}
+
+// The staircase force on one solid cell with fluid neighbours (wall_force_system,
+// crates/cfd_ibm/src/lib.rs:309-395).  The six neighbours are loaded first (in
+// bounds: the boundary ghosts ring the mesh); only the fluid ones are used.
+__device__ __forceinline__ void wall_load3(const Geometry& g, const Physics& ph, const Ibm& ib, const double* q,
+                                           int t, double f[6]) {
     const double gm1 = ph.gamma - 1.0;
-    for (int m = threadIdx.x; m < ib.n_markers; m += FORCE3_THREADS) {
-        const Marker3Dev mk = ib.markers3[m];
-        if (!mk.valid) continue;
-        double img[6];
-        if (!sample_trilinear3(g, ph, q, mk.fluid, mk.lo, mk.t, img)) continue;
-        if (!(isfinite(img[4]) && isfinite(img[5]) && isfinite(img[1]) && isfinite(img[2]) && isfinite(img[3])))
-            continue;
-        const double us[3] = {img[1] - mk.uw[0], img[2] - mk.uw[1], img[3] - mk.uw[2]};
-        const double udotn = us[0] * mk.normal[0] + us[1] * mk.normal[1] + us[2] * mk.normal[2];
-        const double mu = viscosity(ph, img[5]);
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const double ut = us[d] - udotn * mk.normal[d];
-            f[d] += -img[4] * mk.normal[d] * mk.area;
-            f[3 + d] += mu * ut / ib.sample_offset * mk.area;
-        }
-    }
     const double face_area[3] = {g.h[1] * g.h[2], g.h[0] * g.h[2], g.h[0] * g.h[1]};
-    for (int t = threadIdx.x; t < ib.n_ghost; t += FORCE3_THREADS) {
-        const IbmGhost3Dev gh = ib.ghosts3[t];
+    const IbmGhost3Dev gh = ib.ghosts3[t];
+    U5 nb[6];
 #pragma unroll
-        for (int nbk = 0; nbk < 6; ++nbk) {
-            if (!(gh.fluid & (1u << nbk))) continue;
-            const int dim = nbk >> 1;
-            const double sign = (nbk & 1) ? -1.0 : 1.0;
-            const int di = dim == 0 ? (nbk & 1 ? -1 : 1) : 0, dj = dim == 1 ? (nbk & 1 ? -1 : 1) : 0,
-                      dk = dim == 2 ? (nbk & 1 ? -1 : 1) : 0;
-            const U5 uc = load5(q, g.plane, cidx3(g, gh.i + di, gh.j + dj, gh.k + dk));
-            f[6 + dim] -= pressure5(uc, gm1) * sign * face_area[dim];
-            const double inv = 1.0 / uc.r;
-            const double vel[3] = {uc.mx * inv, uc.my * inv, uc.mz * inv};
-            const double ke = 0.5 * uc.r * (vel[0] * vel[0] + vel[1] * vel[1] + vel[2] * vel[2]);
-            const double tt = gm1 * (uc.E - ke) * inv / ph.r_gas;
-            const double mu = viscosity(ph, tt);
-#pragma unroll
-            for (int td = 0; td < 3; ++td)
-                if (td != dim) f[9 + td] += mu * vel[td] / (0.5 * g.h[dim]) * face_area[dim];
-        }
+    for (int n = 0; n < 6; ++n) {
+        const int s = n & 1 ? -1 : 1;
+        nb[n] = load5(q, g.plane, cidx3(g, gh.i + (n < 2 ? s : 0), gh.j + ((n >> 1) == 1 ? s : 0),
+                                        gh.k + (n >= 4 ? s : 0)));
     }
 #pragma unroll
-    for (int v = 0; v < 12; ++v) red[v][threadIdx.x] = f[v];
+    for (int n = 0; n < 6; ++n) {
+        if (!(gh.fluid & (1u << n))) continue;
+        const int dim = n >> 1;
+        const double sign = (n & 1) ? -1.0 : 1.0;
+        const U5 uc = nb[n];
+        f[dim] -= pressure5(uc, gm1) * sign * face_area[dim];
+        const double inv = 1.0 / uc.r;
+        const double vel[3] = {uc.mx * inv, uc.my * inv, uc.mz * inv};
+        const double ke = 0.5 * uc.r * (vel[0] * vel[0] + vel[1] * vel[1] + vel[2] * vel[2]);
+        const double mu = viscosity(ph, gm1 * (uc.E - ke) * inv * ph.inv_r_gas);
+        const double inv_half_dn = 2.0 * g.inv_h[dim];
+#pragma unroll
+        for (int td = 0; td < 3; ++td)
+            if (td != dim) f[3 + td] += mu * vel[td] * inv_half_dn * face_area[dim];
+    }
+}
+
+// The IBM work between two 3-D stage kernels, one launch, as the 2-D
+// ibm_kernel: the first nf blocks integrate the marker (nfm blocks, one marker
+// per thread) and staircase forces of the state q, the others mirror the
+// ghost cells of q.  The two touch disjoint data: the forces read fluid cells,
+// the mirror reads fluid cells and writes solid ones.
+//
+// The forces are bound by latency (2000 markers, a few hundred ghosts): one
+// thread per marker or ghost and one load phase each, block sums in a fixed
+// order, and the last block to finish adds the block sums in a fixed order.
+// One block of 256 threads looping over all of them took 55-58 us per stage at
+// 144x72x72 with 2000 markers, on the step's critical path (165 of about 450 us
+// per step); here they overlap the next mirror and stage.
+//
+// `setup`: thread 0 of the first mirror block does the step's set-up.  The mirror
+// runs whether or not the step does (a run that has reached its stop time still
+// holds mirrored ghosts).  `deferred`: the forces of the previous step's last
+// stage, run only while they are pending, and then cleared by the last block.
+__global__ void __launch_bounds__(IBM_THREADS) ibm3_kernel(Geometry g, Physics ph, Ibm ib, double* q, DevState* st,
+                                                           int nfm, int nf, int setup, int deferred) {
+    pdl_wait_then_release();
+    const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (b >= nf) {  // uniform per block
+        if (setup && b == nf && tid == 0 && st->active) step_setup(ph, st);
+        const int t = (b - nf) * IBM_THREADS + tid;
+        if (t < ib.n_ghost) mirror_ghost3(g, ph, ib, q, t);
+        return;
+    }
+    // Every block reads the flag before it counts itself in; only the last one clears it.
+    if (deferred ? !st->forces_pending : !st->active) return;
+    __shared__ double red[IBM_THREADS / 32][6];
+    __shared__ bool last;
+    double f[6] = {0, 0, 0, 0, 0, 0};
+    const int t = (b < nfm ? b : b - nfm) * IBM_THREADS + tid;
+    if (b < nfm) {
+        if (t < ib.n_markers) marker_load3(g, ph, ib, q, t, f);
+    } else if (t < ib.n_ghost) {
+        wall_load3(g, ph, ib, q, t, f);
+    }
+#pragma unroll
+    for (int d = 0; d < 6; ++d)
+        for (int o = 16; o > 0; o >>= 1) f[d] += __shfl_down_sync(0xffffffffu, f[d], o);
+    if (lane == 0)
+#pragma unroll
+        for (int d = 0; d < 6; ++d) red[warp][d] = f[d];
     __syncthreads();
-    for (int s = FORCE3_THREADS / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s)
+    if (tid == 0) {
 #pragma unroll
-            for (int v = 0; v < 12; ++v) red[v][threadIdx.x] += red[v][threadIdx.x + s];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-        for (int v = 0; v < 12; ++v) ib.force_out[v] = red[v][0];
-        if (ib.history && st->hist_pos < st->hist_cap) {
-            for (int d = 0; d < 6; ++d) ib.history[6 * st->hist_pos + d] = red[d][0];
-            st->hist_pos += 1;
+        for (int d = 0; d < 6; ++d) {
+            double v = red[0][d];
+            for (int w = 1; w < IBM_THREADS / 32; ++w) v += red[w][d];
+            ib.partials[6LL * b + d] = v;
         }
+        __threadfence();
+        last = atomicAdd(ib.counter, 1u) == (unsigned)nf - 1;
     }
+    __syncthreads();
+    if (!last || warp >= 2) return;
+    // warp 0 adds the marker blocks, warp 1 the ghost blocks
+    __threadfence();
+    const volatile double* part = ib.partials;
+    double sum[6] = {0, 0, 0, 0, 0, 0};
+    for (int k = (warp ? nfm : 0) + lane; k < (warp ? nf : nfm); k += 32)
+#pragma unroll
+        for (int d = 0; d < 6; ++d) sum[d] += part[6 * k + d];
+#pragma unroll
+    for (int d = 0; d < 6; ++d)
+        for (int o = 16; o > 0; o >>= 1) sum[d] += __shfl_down_sync(0xffffffffu, sum[d], o);
+    if (lane) return;
+    for (int d = 0; d < 6; ++d) ib.force_out[6 * warp + d] = sum[d];
+    if (warp) return;
+    if (ib.history && st->hist_pos < st->hist_cap) {
+        for (int d = 0; d < 6; ++d) ib.history[6 * st->hist_pos + d] = sum[d];
+        st->hist_pos += 1;
+    }
+    *ib.counter = 0u;  // ready for the next launch
+    if (deferred) st->forces_pending = 0;
 }
 
 // ---- launches ---------------------------------------------------------------
