@@ -7,6 +7,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <string>
 #include <vector>
@@ -99,7 +100,7 @@ struct Net {
 };
 
 // Periodic index for -n <= i < 2n.  Every caller is within 3 cells of the
-// grid (the 5x5 stencil, the residual's neighbours) and every entry point
+// grid (the 5x5 stencil) and every entry point
 // requires nx, ny >= 5, so one conditional wrap replaces an integer modulo
 // (whose division sequence would run per stencil cell).
 __device__ __forceinline__ int wrap(int i, int n) { return i < 0 ? i + n : (i >= n ? i - n : i); }
@@ -126,31 +127,27 @@ struct PaddedState {
     }
 };
 
-// Shared-memory plan of one tile (byte offsets; every operand 128-byte aligned).
-constexpr int SM_X = 0;                       // [128][K1]   A of layer 1
-constexpr int SM_XT = SM_X + 128 * K1 * 2;    // [K1][128]   B of dW1
-constexpr int SM_W1 = SM_XT + K1 * 128 * 2;   // [H][K1]
-constexpr int SM_W2 = SM_W1 + H * K1 * 2;     // [H][H]
-constexpr int SM_W3 = SM_W2 + H * H * 2;      // [N3][H]
-constexpr int SM_W2T = SM_W3 + N3 * H * 2;    // [H][H]      W2 transposed
-constexpr int SM_W3T = SM_W2T + H * H * 2;    // [H][N3]     W3 transposed
-constexpr int SM_H1 = SM_W3T + H * N3 * 2;    // [128][H]
-constexpr int SM_H2 = SM_H1 + 128 * H * 2;    // [128][H]
-constexpr int SM_H1T = SM_H2 + 128 * H * 2;   // [H][128]
-constexpr int SM_H2T = SM_H1T + H * 128 * 2;  // [H][128]
-constexpr int SM_DY = SM_H2T + H * 128 * 2;   // [128][N3]   output gradient
-constexpr int SM_DZ = SM_DY + 128 * N3 * 2;   // [128][H]    dZ2, A of dH1
-constexpr int SM_AT = SM_DZ + 128 * H * 2;    // [128][128]  transposed gradient, A of the weight gradients
-constexpr int SM_RED = SM_AT + 128 * 128 * 2; // [4][K1] floats: per-warp column sums
-constexpr int SM_TOTAL = SM_RED + 4 * K1 * 4;
-constexpr int SM_FWD = SM_H2 + 128 * H * 2;   // the forward pass needs the buffers up to H2
-
-__device__ __forceinline__ void put(unsigned char* base, int r, int k, int rows, float v) {
-    *reinterpret_cast<__nv_bfloat16*>(base + tc::canon_offset(r, k, rows)) = __float2bfloat16_rn(v);
-}
-__device__ __forceinline__ float get_bf(const unsigned char* base, int r, int k, int rows) {
-    return __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(base + tc::canon_offset(r, k, rows)));
-}
+// Shared-memory plans (byte offsets; every operand 128-byte aligned).  Forward:
+// the hidden activations overwrite X, which the first product has read by then.
+constexpr int X_BYTES = 128 * K1 * 2, H_BYTES = 128 * H * 2, ONE_BYTES = 128 * 8 * 2;
+constexpr int W_BYTES = (H * K1 + H * H + N3 * H) * 2;
+constexpr int FW_X = 0, FW_H1 = 0, FW_H2 = H_BYTES, FW_W = X_BYTES;
+constexpr int SM_FWD = FW_W + W_BYTES;                  // 38.9 KB
+// Backward: a column of ones follows H1 and H2 (and stands in X's padding), so
+// that the weight gradients' products also form the bias gradients.  dZ1
+// overwrites H2 once dW3 has read it.  A transposed operand of M = 128 spans 16
+// core-matrix columns (32 KB): X, H1 and H2 each have that much after them,
+// and what lies past their own columns only reaches accumulator rows that
+// nobody reads.
+constexpr int BW_X = 0, BW_H1 = BW_X + X_BYTES, BW_ONE1 = BW_H1 + H_BYTES, BW_H2 = BW_ONE1 + ONE_BYTES,
+              BW_ONE2 = BW_H2 + H_BYTES, BW_DZ2 = BW_ONE2 + ONE_BYTES, BW_DY = BW_DZ2 + H_BYTES,
+              BW_W = BW_DY + 128 * N3 * 2, BW_DZ1 = BW_H2;
+constexpr int SM_BWD = BW_W + W_BYTES;                  // 71.7 KB
+static_assert(BW_H2 + 16 * 2048 <= SM_BWD, "transposed operands stay inside the block's shared memory");
+// Resident blocks per SM (shared memory and 512 tensor-memory columns: 5 x 32, 3 x 128)
+constexpr int FWD_BLOCKS = 5, BWD_BLOCKS = 3;
+constexpr uint32_t FWD_COLS = 32, BWD_COLS = 128;
+constexpr uint32_t T_D = 0, T_DW1 = 32, T_DW2 = 64, T_DW3 = 96;  // accumulator columns (backward)
 
 struct FaceId {
     int b, orient, i, j;
@@ -201,8 +198,16 @@ struct PrimView {
     }
 };
 
+// Programmatic dependent launch, as the step's other kernels (efvm_kernels.cu):
+// nothing a predecessor wrote is read before the wait.
+__device__ __forceinline__ void pdl_wait_then_release() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 template <class SV>
 __global__ void nn_prims_kernel(SV sv, int batch, float gamma, float4* __restrict__ out) {
+    pdl_wait_then_release();
     const long long n = (long long)sv.nx * sv.ny, total = (long long)batch * n;
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
         const int b = (int)(t / n);
@@ -220,133 +225,138 @@ __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
 }
 
 // The stencil features of face `id`, written as row r of X with one 16-byte
-// store per two stencil cells (8 consecutive K in the canonical layout), and
-// into X^T (element by element) when xt != null.  Feature 4q + v is variable v
-// (rho - 1, normal velocity, tangential velocity, p - 1) of stencil cell
-// q = (c + 2) * 5 + (a + 3), a the offset along the face normal (-3..1), c across.
-__device__ void gather_face(const PrimView& pv, const FaceId& id, unsigned char* x, unsigned char* xt, int r) {
-#pragma unroll 7
+// store per two stencil cells (8 consecutive K in the canonical layout).
+// Feature 4q + v is variable v (rho - 1, normal velocity, tangential velocity,
+// p - 1) of stencil cell q = (c + 2) * 5 + (a + 3), a the offset along the face
+// normal (-3..1), c across.  Feature IN is `one` (a column of ones gives the
+// backward pass its bias gradients; the weights of the padding are zero).
+__device__ __forceinline__ void gather_face(const PrimView& pv, const FaceId& id, unsigned char* x, int r, float one) {
+    // the wrapped offsets of the five cells along and across the normal
+    int along[5], across[5];
+    const int n_al = id.orient == 0 ? pv.nx : pv.ny, n_ac = id.orient == 0 ? pv.ny : pv.nx;
+    const int s_al = id.orient == 0 ? 1 : pv.nx, s_ac = id.orient == 0 ? pv.nx : 1;
+    const int p_al = id.orient == 0 ? id.i : id.j, p_ac = id.orient == 0 ? id.j : id.i;
+#pragma unroll
+    for (int k = 0; k < 5; ++k) {
+        along[k] = wrap(p_al + k - 3, n_al) * s_al;
+        across[k] = wrap(p_ac + k - 2, n_ac) * s_ac;
+    }
+    const float4* base = pv.p + (long long)id.b * pv.ny * pv.nx;
+#pragma unroll
     for (int m = 0; m < K1 / 8; ++m) {
         float f[8];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int q = 2 * m + h;
             if (q < 25) {
-                const int c = q / 5 - 2, a = q % 5 - 3;
-                const int ci = id.orient == 0 ? id.i + a : id.i + c;
-                const int cj = id.orient == 0 ? id.j + c : id.j + a;
-                const float4 w = pv.get(id.b, ci, cj);
+                const float4 w = base[across[q / 5] + along[q % 5]];
                 f[4 * h + 0] = w.x;
                 f[4 * h + 1] = id.orient == 0 ? w.y : w.z;
                 f[4 * h + 2] = id.orient == 0 ? w.z : w.y;
                 f[4 * h + 3] = w.w;
             } else {
-                f[4 * h + 0] = f[4 * h + 1] = f[4 * h + 2] = f[4 * h + 3] = 0.f;
+                f[4 * h + 0] = q == 25 ? one : 0.f;
+                f[4 * h + 1] = f[4 * h + 2] = f[4 * h + 3] = 0.f;
             }
         }
-        const uint4 v = make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]),
-                                   pack_bf16x2(f[6], f[7]));
-        *reinterpret_cast<uint4*>(x + tc::canon_offset(r, 8 * m, 128)) = v;
-        if (xt)
-#pragma unroll
-            for (int e = 0; e < 8; ++e) put(xt, 8 * m + e, r, K1, f[e]);
+        *reinterpret_cast<uint4*>(x + tc::canon_offset(r, 8 * m, 128)) =
+            make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]),
+                       pack_bf16x2(f[6], f[7]));
     }
 }
 
-// Weights into shared memory, 16 bytes (8 consecutive K of one row) per copy,
-// and their transposes for the backward pass element by element.
-__device__ void load_weights(const Net& net, unsigned char* sm, bool transposed) {
+// Weights into shared memory at w (W1, W2, W3), 16 bytes (8 consecutive K of one row) per copy.
+constexpr int W2_OFF = H * K1 * 2, W3_OFF = W2_OFF + H * H * 2;
+__device__ __forceinline__ void load_weights(const Net& net, unsigned char* w) {
     const uint4* w1 = reinterpret_cast<const uint4*>(net.w1);
     for (int t = threadIdx.x; t < H * K1 / 8; t += blockDim.x) {
         const int o = t / (K1 / 8), g = t - o * (K1 / 8);
-        *reinterpret_cast<uint4*>(sm + SM_W1 + tc::canon_offset(o, 8 * g, H)) = w1[t];
+        *reinterpret_cast<uint4*>(w + tc::canon_offset(o, 8 * g, H)) = w1[t];
     }
     const uint4* w2 = reinterpret_cast<const uint4*>(net.w2);
     for (int t = threadIdx.x; t < H * H / 8; t += blockDim.x) {
         const int o = t / (H / 8), g = t - o * (H / 8);
-        *reinterpret_cast<uint4*>(sm + SM_W2 + tc::canon_offset(o, 8 * g, H)) = w2[t];
+        *reinterpret_cast<uint4*>(w + W2_OFF + tc::canon_offset(o, 8 * g, H)) = w2[t];
     }
     const uint4* w3 = reinterpret_cast<const uint4*>(net.w3);
     for (int t = threadIdx.x; t < N3 * H / 8; t += blockDim.x) {
         const int o = t / (H / 8), g = t - o * (H / 8);
-        *reinterpret_cast<uint4*>(sm + SM_W3 + tc::canon_offset(o, 8 * g, N3)) = w3[t];
-    }
-    if (transposed) {
-        for (int t = threadIdx.x; t < H * H; t += blockDim.x) {
-            const int o = t / H, k = t - o * H;
-            *reinterpret_cast<__nv_bfloat16*>(sm + SM_W2T + tc::canon_offset(k, o, H)) = net.w2[t];
-        }
-        for (int t = threadIdx.x; t < N3 * H; t += blockDim.x) {
-            const int o = t / H, k = t - o * H;
-            *reinterpret_cast<__nv_bfloat16*>(sm + SM_W3T + tc::canon_offset(k, o, H)) = net.w3[t];
-        }
+        *reinterpret_cast<uint4*>(w + W3_OFF + tc::canon_offset(o, 8 * g, N3)) = w3[t];
     }
 }
 
-// Tensor-core state of a tile: TMEM columns, the mbarrier and its phase.
+// Tensor-core state of a block: its tensor memory, the mbarrier and its phase.
 struct TC {
     uint64_t* bar;
     uint32_t tmem;
     uint32_t phase;
-    bool ok;
 };
 
-// Issue D = A B^T, wait for it (bounded) and make TMEM readable; false if the
-// wait ran out anywhere in the CTA.
-__device__ bool run_gemm(TC& t, const unsigned char* a, const unsigned char* b, int n, int k) {
+// Shared-memory operands written so far become visible to the tensor core, and
+// its accumulators read so far may be overwritten.
+__device__ __forceinline__ void publish() {
     tc::fence_smem_to_async();
     tc::fence_before_sync();
     __syncthreads();
-    tc::gemm_issue(t.tmem, a, b, n, k, t.bar);
+}
+// Wait (bounded) for the products committed last and make their accumulators
+// readable; false if the wait ran out anywhere in the block.
+__device__ __forceinline__ bool products_done(TC& t) {
     bool ok = tc::mbar_wait(t.bar, t.phase);
     ok = __syncthreads_and(ok);
     t.phase ^= 1u;
     if (!ok) {
         if (threadIdx.x == 0) atomicExch(&g_nn_error, 1);
         tc::mbar_wait(t.bar, t.phase ^ 1u);  // a second bounded chance to retire before TMEM is released
-        t.ok = false;
         return false;
     }
     tc::fence_after_sync();
     return true;
 }
 
-// Row r's 32 accumulator columns + bias, through relu, into A (row r) and, if
-// given, its transpose.  Returns nothing; the caller barriers before reuse.
-__device__ void relu_epilogue(uint32_t tmem, const float* bias, unsigned char* out, unsigned char* out_t, int r) {
+// D = A B^T of K-major operands (A 128 rows, B n rows), committed.
+__device__ __forceinline__ bool run_gemm(TC& t, const unsigned char* a, const unsigned char* b, int n, int k) {
+    publish();
+    tc::gemm_issue(t.tmem, a, b, n, k, t.bar);
+    return products_done(t);
+}
+
+// 32 consecutive FP32 values as a row of 32 BF16 in the canonical layout.
+__device__ __forceinline__ void store_row(unsigned char* out, int r, const float (&v)[H]) {
+#pragma unroll
+    for (int g = 0; g < H / 8; ++g)
+        *reinterpret_cast<uint4*>(out + tc::canon_offset(r, 8 * g, 128)) =
+            make_uint4(pack_bf16x2(v[8 * g], v[8 * g + 1]), pack_bf16x2(v[8 * g + 2], v[8 * g + 3]),
+                       pack_bf16x2(v[8 * g + 4], v[8 * g + 5]), pack_bf16x2(v[8 * g + 6], v[8 * g + 7]));
+}
+// Accumulator row r (32 columns).
+__device__ __forceinline__ void load_row(uint32_t tmem, float (&v)[H]) {
 #pragma unroll
     for (int c0 = 0; c0 < H; c0 += 16) {
-        float v[16];
-        tc::tmem_ld16(tmem, c0, v);
+        float q[16];
+        tc::tmem_ld16(tmem, c0, q);
 #pragma unroll
-        for (int c = 0; c < 16; ++c) v[c] = fmaxf(v[c] + bias[c0 + c], 0.f);
-#pragma unroll
-        for (int g = 0; g < 2; ++g)
-            *reinterpret_cast<uint4*>(out + tc::canon_offset(r, c0 + 8 * g, 128)) =
-                make_uint4(pack_bf16x2(v[8 * g], v[8 * g + 1]), pack_bf16x2(v[8 * g + 2], v[8 * g + 3]),
-                           pack_bf16x2(v[8 * g + 4], v[8 * g + 5]), pack_bf16x2(v[8 * g + 6], v[8 * g + 7]));
-        if (out_t)
-#pragma unroll
-            for (int c = 0; c < 16; ++c) put(out_t, c0 + c, r, H, v[c]);
+        for (int c = 0; c < 16; ++c) v[c0 + c] = q[c];
     }
 }
-
-// Forward pass of one tile through layer 2 (H1, H2 in shared memory).
-__device__ bool forward_hidden(const PrimView& pv, const Net& net, unsigned char* sm, TC& t, long long f0,
-                               bool keep_transposes) {
-    const int r = threadIdx.x;
-    const FaceId id = face_of(f0 + r, pv.nx, pv.ny);
-    gather_face(pv, id, sm + SM_X, keep_transposes ? sm + SM_XT : nullptr, r);
-    load_weights(net, sm, keep_transposes);
-    if (!run_gemm(t, sm + SM_X, sm + SM_W1, H, K1)) return false;
-    relu_epilogue(t.tmem, net.p + P_B1, sm + SM_H1, keep_transposes ? sm + SM_H1T : nullptr, r);
-    if (!run_gemm(t, sm + SM_H1, sm + SM_W2, H, H)) return false;
-    relu_epilogue(t.tmem, net.p + P_B2, sm + SM_H2, keep_transposes ? sm + SM_H2T : nullptr, r);
-    return true;
+// Row r's accumulator + bias through relu into row r of `out`; bit c of the
+// result is set where unit c is active.
+__device__ __forceinline__ uint32_t relu_epilogue(uint32_t tmem, const float* bias, unsigned char* out, int r) {
+    float v[H];
+    load_row(tmem, v);
+    uint32_t on = 0;
+#pragma unroll
+    for (int c = 0; c < H; ++c) {
+        v[c] = fmaxf(v[c] + bias[c], 0.f);
+        // the activity of the value that is stored, rounded to BF16
+        on |= (__bfloat162float(__float2bfloat16_rn(v[c])) > 0.f ? 1u : 0u) << c;
+    }
+    store_row(out, r, v);
+    return on;
 }
 
-__device__ void tile_setup(TC& t, uint64_t* bar, uint32_t* slot) {
-    if ((threadIdx.x >> 5) == 0) tc::tmem_alloc(slot, 128);
+__device__ __forceinline__ void tile_setup(TC& t, uint64_t* bar, uint32_t* slot, uint32_t cols) {
+    if ((threadIdx.x >> 5) == 0) tc::tmem_alloc(slot, cols);
     if (threadIdx.x == 0) tc::mbar_init(bar, 1);
     tc::fence_before_sync();
     __syncthreads();
@@ -354,33 +364,46 @@ __device__ void tile_setup(TC& t, uint64_t* bar, uint32_t* slot) {
     t.bar = bar;
     t.tmem = *slot;
     t.phase = 0;
-    t.ok = true;
 }
-__device__ void tile_teardown(const TC& t) {
+__device__ __forceinline__ void tile_teardown(const TC& t, uint32_t cols) {
     tc::fence_before_sync();
     __syncthreads();
-    if ((threadIdx.x >> 5) == 0) tc::tmem_free(t.tmem, 128);
+    if ((threadIdx.x >> 5) == 0) tc::tmem_free(t.tmem, cols);
 }
 
 // Forward: the correction of every face, grid frame, corr[((b*2+orient)*4+v)*ny*nx + j*nx + i].
 // sensor > 0 (inference): a face whose two cells differ in pressure by more than
 // sensor * min(p), or where rho or p is not positive, keeps the plain flux.
-__global__ void __launch_bounds__(128) nn_forward_kernel(PrimView pv, Net net, float* __restrict__ corr, float sensor,
-                                                         unsigned long long* fallbacks) {
+//
+// Bound by the latency of a tile's chain (gather 25 cells, three products and
+// their read-backs), so the blocks are persistent (weights and tensor memory
+// set up once) and small enough for five per SM, whose tiles overlap.  One
+// 87 KB block per tile, two resident, took 51 us for 262144 faces (2048 tiles).
+__global__ void __launch_bounds__(128) nn_forward_kernel(PrimView pv, Net net, int tiles, float* __restrict__ corr,
+                                                         float sensor, unsigned long long* fallbacks) {
     extern __shared__ __align__(128) unsigned char sm[];
     __shared__ __align__(8) uint64_t bar;
     __shared__ uint32_t slot;
+    __shared__ float bias[2 * H + NOUT];
     TC t;
-    tile_setup(t, &bar, &slot);
-    const long long f0 = (long long)blockIdx.x * 128;
     const int r = threadIdx.x;
-    if (forward_hidden(pv, net, sm, t, f0, false) && run_gemm(t, sm + SM_H2, sm + SM_W3, N3, H)) {
+    load_weights(net, sm + FW_W);
+    if (r < 2 * H + NOUT) bias[r] = net.p[P_B1 + r];  // b1, b2, b3 are consecutive
+    tile_setup(t, &bar, &slot, FWD_COLS);
+    pdl_wait_then_release();
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const FaceId id = face_of((long long)tile * 128 + r, pv.nx, pv.ny);
+        gather_face(pv, id, sm + FW_X, r, 0.f);
+        if (!run_gemm(t, sm + FW_X, sm + FW_W, H, K1)) break;
+        relu_epilogue(t.tmem, bias, sm + FW_H1, r);
+        if (!run_gemm(t, sm + FW_H1, sm + FW_W + W2_OFF, H, H)) break;
+        relu_epilogue(t.tmem, bias + H, sm + FW_H2, r);
+        if (!run_gemm(t, sm + FW_H2, sm + FW_W + W3_OFF, N3, H)) break;
         float v[16];
         tc::tmem_ld16(t.tmem, 0, v);
-        const FaceId id = face_of(f0 + r, pv.nx, pv.ny);
         float y[4];
 #pragma unroll
-        for (int o = 0; o < 4; ++o) y[o] = (v[o] + net.p[P_B3 + o]) * net.out_scale;
+        for (int o = 0; o < 4; ++o) y[o] = (v[o] + bias[2 * H + o]) * net.out_scale;
         if (sensor > 0.f) {
             const int il = id.orient == 0 ? id.i - 1 : id.i, jl = id.orient == 0 ? id.j : id.j - 1;
             const float4 ql = pv.get(id.b, il, jl), qr = pv.get(id.b, id.i, id.j);
@@ -398,180 +421,200 @@ __global__ void __launch_bounds__(128) nn_forward_kernel(PrimView pv, Net net, f
 #pragma unroll
         for (int q = 0; q < 4; ++q) corr[((long long)(id.b * 2 + id.orient) * 4 + q) * nn + cell] = g[q];
     }
-    tile_teardown(t);
-}
-
-// Column sums of per-thread rows: each warp reduces its 32 rows by shuffles,
-// then thread c adds the four warp sums in order (deterministic).
-__device__ void column_sums(const float* vals, int ncols, float* red, float* out) {
-    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int c = 0; c < ncols; ++c) {
-        float s = vals[c];
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) red[w * K1 + c] = s;
-    }
-    __syncthreads();
-    if ((int)threadIdx.x < ncols) out[threadIdx.x] = red[threadIdx.x] + red[K1 + threadIdx.x] + red[2 * K1 + threadIdx.x] + red[3 * K1 + threadIdx.x];
-    __syncthreads();
-}
-
-// Rows 0..rows-1 of the accumulator (warp 0's lanes), ncols columns, to out[row * ncols + col].
-__device__ void store_weight_grad(uint32_t tmem, int rows, int ncols, float* out) {
-    if ((threadIdx.x >> 5) != 0) return;  // warp-uniform: rows < 32 live in warp 0's lanes
-    const int lane = threadIdx.x & 31;
-    for (int c0 = 0; c0 < ncols; c0 += 16) {
-        float v[16];
-        tc::tmem_ld16(tmem, c0, v);
-        if (lane < rows)
-#pragma unroll
-            for (int c = 0; c < 16; ++c)
-                if (c0 + c < ncols) out[lane * ncols + c0 + c] = v[c];
-    }
+    tile_teardown(t, FWD_COLS);
 }
 
 // Backward: given dL/dcorr (grid frame, the layout of corr), the gradient of the
-// loss with respect to every parameter, summed over this tile's 128 faces, into
-// partials[tile][P_COUNT].
-__global__ void __launch_bounds__(128) nn_backward_kernel(PrimView sv, Net net, const float* __restrict__ dcorr,
+// loss with respect to every parameter, summed over the block's tiles, into
+// partials[block][P_COUNT].
+//
+// Per tile four product phases form the chain: X W1^T; H1 W2^T; dZ2 W2 (beside
+// dW3 += H2^T dY and dW2 += H1^T dZ2); dW1 += X^T dZ1.  The weight gradients
+// are kept as their transposes, features along M, and stay in tensor memory over
+// all of a block's tiles; their operands are the forward buffers read MN-major,
+// so nothing is stored twice or transposed.  dH2 = dY W3 has K = 4 and runs on
+// the FP32 units.  One block per tile with stored transposes (150 KB, one block
+// per SM), shuffled column sums for the biases and 39 MB of per-tile partials
+// took 235 us and 84 us for their sum at 262144 faces.
+__global__ void __launch_bounds__(128) nn_backward_kernel(PrimView pv, Net net, int tiles,
+                                                          const float* __restrict__ dcorr,
                                                           float* __restrict__ partials) {
     extern __shared__ __align__(128) unsigned char sm[];
     __shared__ __align__(8) uint64_t bar;
     __shared__ uint32_t slot;
+    __shared__ float bias[2 * H];
+    __shared__ float4 w3[H];  // column c of W3
     TC t;
-    tile_setup(t, &bar, &slot);
-    const long long f0 = (long long)blockIdx.x * 128;
     const int r = threadIdx.x;
-    float* part = partials + (long long)blockIdx.x * P_COUNT;
-    float* red = reinterpret_cast<float*>(sm + SM_RED);
-    // the transposed-gradient operand: rows beyond the layer width stay zero
-    for (int q = threadIdx.x; q < 128 * 128 * 2 / 16; q += blockDim.x)
-        reinterpret_cast<uint4*>(sm + SM_AT)[q] = make_uint4(0, 0, 0, 0);
-    do {
-        if (!forward_hidden(sv, net, sm, t, f0, true)) break;
-        // output gradient of this face in its own frame, times out_scale
-        const FaceId id = face_of(f0 + r, sv.nx, sv.ny);
-        const long long cell = (long long)id.j * sv.nx + id.i, nn = (long long)sv.nx * sv.ny;
+    load_weights(net, sm + BW_W);
+    if (r < 2 * H) bias[r] = net.p[P_B1 + r];
+    if (r < H)
+        w3[r] = make_float4(__bfloat162float(net.w3[r]), __bfloat162float(net.w3[H + r]),
+                            __bfloat162float(net.w3[2 * H + r]), __bfloat162float(net.w3[3 * H + r]));
+    {
+        const uint4 ones = make_uint4(pack_bf16x2(1.f, 0.f), 0u, 0u, 0u);
+        *reinterpret_cast<uint4*>(sm + BW_ONE1 + tc::canon_offset(r, 0, 128)) = ones;
+        *reinterpret_cast<uint4*>(sm + BW_ONE2 + tc::canon_offset(r, 0, 128)) = ones;
+    }
+    tile_setup(t, &bar, &slot, BWD_COLS);
+    const uint32_t idesc_t = tc::idesc_bf16_f32(128, H) | tc::A_MN | tc::B_MN;
+    bool ok = true, first = true;
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const FaceId id = face_of((long long)tile * 128 + r, pv.nx, pv.ny);
+        // output gradient of this face in its own frame, times out_scale, as BF16
+        const long long cell = (long long)id.j * pv.nx + id.i, nn = (long long)pv.nx * pv.ny;
         float g[4];
 #pragma unroll
         for (int q = 0; q < 4; ++q) g[q] = dcorr[((long long)(id.b * 2 + id.orient) * 4 + q) * nn + cell];
-        const float dy[4] = {g[0] * net.out_scale, (id.orient == 0 ? g[1] : g[2]) * net.out_scale,
-                             (id.orient == 0 ? g[2] : g[1]) * net.out_scale, g[3] * net.out_scale};
-        float dyrow[N3];
+        const float dyf[4] = {g[0] * net.out_scale, (id.orient == 0 ? g[1] : g[2]) * net.out_scale,
+                              (id.orient == 0 ? g[2] : g[1]) * net.out_scale, g[3] * net.out_scale};
+        float dy[4];
 #pragma unroll
-        for (int o = 0; o < N3; ++o) dyrow[o] = o < NOUT ? __bfloat162float(__float2bfloat16_rn(dy[o])) : 0.f;
+        for (int o = 0; o < 4; ++o) dy[o] = __bfloat162float(__float2bfloat16_rn(dyf[o]));
+        gather_face(pv, id, sm + BW_X, r, 1.f);
+        *reinterpret_cast<uint4*>(sm + BW_DY + tc::canon_offset(r, 0, 128)) =
+            make_uint4(pack_bf16x2(dy[0], dy[1]), pack_bf16x2(dy[2], dy[3]), 0u, 0u);
+        *reinterpret_cast<uint4*>(sm + BW_DY + tc::canon_offset(r, 8, 128)) = make_uint4(0u, 0u, 0u, 0u);
+        if (!(ok = run_gemm(t, sm + BW_X, sm + BW_W, H, K1))) break;
+        const uint32_t on1 = relu_epilogue(t.tmem + T_D, bias, sm + BW_H1, r);
+        if (!(ok = run_gemm(t, sm + BW_H1, sm + BW_W + W2_OFF, H, H))) break;
+        const uint32_t on2 = relu_epilogue(t.tmem + T_D, bias + H, sm + BW_H2, r);
+        float dz[H];
+        // dZ2 = (dY W3) * relu'(h2)
 #pragma unroll
-        for (int g = 0; g < 2; ++g)
-            *reinterpret_cast<uint4*>(sm + SM_DY + tc::canon_offset(r, 8 * g, 128)) =
-                make_uint4(pack_bf16x2(dyrow[8 * g], dyrow[8 * g + 1]), pack_bf16x2(dyrow[8 * g + 2], dyrow[8 * g + 3]),
-                           pack_bf16x2(dyrow[8 * g + 4], dyrow[8 * g + 5]), pack_bf16x2(dyrow[8 * g + 6], dyrow[8 * g + 7]));
-#pragma unroll
-        for (int o = 0; o < NOUT; ++o) put(sm + SM_AT, o, r, 128, dyrow[o]);
-        column_sums(dyrow, NOUT, red, part + P_B3);
-        // dW3 = dY^T H2
-        if (!run_gemm(t, sm + SM_AT, sm + SM_H2T, H, 128)) break;
-        store_weight_grad(t.tmem, NOUT, H, part + P_W3);
-        // dH2 = dY W3, dZ2 = dH2 * relu'(h2)
-        if (!run_gemm(t, sm + SM_DY, sm + SM_W3T, H, N3)) break;
-        {
-            float dz[H];
-#pragma unroll
-            for (int c0 = 0; c0 < H; c0 += 16) {
-                float v[16];
-                tc::tmem_ld16(t.tmem, c0, v);
-#pragma unroll
-                for (int c = 0; c < 16; ++c) {
-                    const float z = get_bf(sm + SM_H2, r, c0 + c, 128) > 0.f ? v[c] : 0.f;
-                    dz[c0 + c] = __bfloat162float(__float2bfloat16_rn(z));
-                }
-            }
-#pragma unroll
-            for (int g = 0; g < H / 8; ++g)
-                *reinterpret_cast<uint4*>(sm + SM_DZ + tc::canon_offset(r, 8 * g, 128)) =
-                    make_uint4(pack_bf16x2(dz[8 * g], dz[8 * g + 1]), pack_bf16x2(dz[8 * g + 2], dz[8 * g + 3]),
-                               pack_bf16x2(dz[8 * g + 4], dz[8 * g + 5]), pack_bf16x2(dz[8 * g + 6], dz[8 * g + 7]));
-#pragma unroll
-            for (int c = 0; c < H; ++c) put(sm + SM_AT, c, r, 128, dz[c]);
-            column_sums(dz, H, red, part + P_B2);
+        for (int c = 0; c < H; ++c) {
+            const float4 w = w3[c];
+            const float v = fmaf(dy[3], w.w, fmaf(dy[2], w.z, fmaf(dy[1], w.y, dy[0] * w.x)));
+            dz[c] = (on2 >> c) & 1u ? v : 0.f;
         }
-        // dW2 = dZ2^T H1
-        if (!run_gemm(t, sm + SM_AT, sm + SM_H1T, H, 128)) break;
-        store_weight_grad(t.tmem, H, H, part + P_W2);
-        // dH1 = dZ2 W2, dZ1 = dH1 * relu'(h1)
-        if (!run_gemm(t, sm + SM_DZ, sm + SM_W2T, H, H)) break;
-        {
-            float dz[H];
-#pragma unroll
-            for (int c0 = 0; c0 < H; c0 += 16) {
-                float v[16];
-                tc::tmem_ld16(t.tmem, c0, v);
-#pragma unroll
-                for (int c = 0; c < 16; ++c) {
-                    const float z = get_bf(sm + SM_H1, r, c0 + c, 128) > 0.f ? v[c] : 0.f;
-                    dz[c0 + c] = __bfloat162float(__float2bfloat16_rn(z));
-                }
-            }
-            __syncthreads();  // the previous GEMM has read A^T; now overwrite it
-#pragma unroll
-            for (int c = 0; c < H; ++c) put(sm + SM_AT, c, r, 128, dz[c]);
-            column_sums(dz, H, red, part + P_B1);
+        store_row(sm + BW_DZ2, r, dz);
+        publish();
+        if (threadIdx.x == 0) {
+            tc::fence_after_sync();
+            // dW3^T += H2^T dY, D = dZ2 W2 (both before the commit: dZ1 overwrites H2), then dW2^T += H1^T dZ2
+            tc::mma_steps(t.tmem + T_DW3, sm + BW_H2, 128, 2048, 256, sm + BW_DY, 128, 2048, 256,
+                          tc::idesc_bf16_f32(128, N3) | tc::A_MN | tc::B_MN, 8, !first);
+            tc::mma_steps(t.tmem + T_D, sm + BW_DZ2, 2048, 128, 4096, sm + BW_W + W2_OFF, 128, 16 * H, 256,
+                          tc::idesc_bf16_f32(128, H) | tc::B_MN, H / 16, false);
+            tc::mma_commit(t.bar);
+            tc::mma_steps(t.tmem + T_DW2, sm + BW_H1, 128, 2048, 256, sm + BW_DZ2, 128, 2048, 256, idesc_t, 8, !first);
         }
-        // dW1 = dZ1^T X
-        if (!run_gemm(t, sm + SM_AT, sm + SM_XT, K1, 128)) break;
-        store_weight_grad(t.tmem, H, K1, part + P_W1);
-    } while (0);
-    tile_teardown(t);
+        if (!(ok = products_done(t))) break;
+        // dZ1 = D * relu'(h1)
+        load_row(t.tmem + T_D, dz);
+#pragma unroll
+        for (int c = 0; c < H; ++c) dz[c] = (on1 >> c) & 1u ? dz[c] : 0.f;
+        store_row(sm + BW_DZ1, r, dz);
+        publish();
+        if (threadIdx.x == 0) {
+            tc::fence_after_sync();
+            tc::mma_steps(t.tmem + T_DW1, sm + BW_X, 128, 2048, 256, sm + BW_DZ1, 128, 2048, 256, idesc_t, 8, !first);
+            tc::mma_commit(t.bar);
+        }
+        first = false;
+        if (!(ok = products_done(t))) break;
+    }
+    if (ok) {
+        // row k of the transposed gradients is feature k; the row of ones holds the biases
+        float* part = partials + (long long)blockIdx.x * P_COUNT;
+        float v[H];
+        load_row(t.tmem + T_DW1, v);
+        if (r < K1)
+#pragma unroll
+            for (int o = 0; o < H; ++o) part[P_W1 + o * K1 + r] = r < IN ? v[o] : 0.f;
+        if (r == IN)
+#pragma unroll
+            for (int o = 0; o < H; ++o) part[P_B1 + o] = v[o];
+        load_row(t.tmem + T_DW2, v);
+        if (r < H)
+#pragma unroll
+            for (int o = 0; o < H; ++o) part[P_W2 + o * H + r] = v[o];
+        if (r == H)
+#pragma unroll
+            for (int o = 0; o < H; ++o) part[P_B2 + o] = v[o];
+        float u[16];
+        tc::tmem_ld16(t.tmem + T_DW3, 0, u);
+        if (r < H)
+#pragma unroll
+            for (int o = 0; o < NOUT; ++o) part[P_W3 + o * H + r] = u[o];
+        if (r == H)
+#pragma unroll
+            for (int o = 0; o < NOUT; ++o) part[P_B3 + o] = u[o];
+    }
+    tile_teardown(t, BWD_COLS);
 }
 
-// grad[p] = sum over tiles of partials[tile][p], in tile order.
-__global__ void nn_reduce_kernel(const float* __restrict__ partials, int tiles, float* __restrict__ grad) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= P_COUNT) return;
+// grad[p] = sum over blocks of partials[block][p], in a fixed order: a warp per
+// slice of the blocks over 32 parameters, then the slices in order.  The grid's
+// first thread also passes the loss on with the tensor-core status beside it,
+// so that the host reads both with one copy.  (One thread per parameter over
+// 2048 per-tile partials took 84 us: 19 blocks of serial loads.)
+constexpr int RED_SLICES = 8;
+__global__ void __launch_bounds__(32 * RED_SLICES) nn_reduce_kernel(const float* __restrict__ partials, int blocks,
+                                                                    float* __restrict__ grad,
+                                                                    float* __restrict__ grad_out, double* loss) {
+    __shared__ float sum[RED_SLICES][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int p = blockIdx.x * 32 + lane;
     float s = 0.f;
-    for (int t = 0; t < tiles; ++t) s += partials[(long long)t * P_COUNT + p];
-    grad[p] = s;
+    if (p < P_COUNT)
+#pragma unroll 8
+        for (int b = w; b < blocks; b += RED_SLICES) s += partials[(long long)b * P_COUNT + p];
+    sum[w][lane] = s;
+    __syncthreads();
+    if (w == 0 && p < P_COUNT) {
+        for (int k = 1; k < RED_SLICES; ++k) s += sum[k][lane];
+        grad[p] = s;
+        if (grad_out) grad_out[p] = s;
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) loss[1] = (double)g_nn_error;
 }
 
 // Residual loss of a batch: e = R + div(corr) per cell and variable,
-// L = sum_v w_v * mean(e_v^2); dcorr = dL/dcorr.  One thread per cell.
-__global__ void nn_residual_kernel(const float* __restrict__ corr, const double* __restrict__ resid, int batch, int nx,
-                                   int ny, double inv_dx, double inv_dy, float w0, float w1, float w2, float w3,
-                                   float* __restrict__ dcorr, double* loss) {
+// L = sum_v w_v * mean(e_v^2); dcorr = dL/dcorr.  One thread per cell; the
+// loss goes out with one atomic per block (one per warp serialised on the one
+// address: 13.4 us at 131072 cells).
+__global__ void __launch_bounds__(256) nn_residual_kernel(const float* __restrict__ corr,
+                                                          const double* __restrict__ resid, int batch, int nx, int ny,
+                                                          double inv_dx, double inv_dy, float w0, float w1, float w2,
+                                                          float w3, float* __restrict__ dcorr, double* loss) {
+    __shared__ double red[8];
     const long long n = (long long)nx * ny, total = (long long)batch * n;
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     double l = 0.0;
     if (t < total) {
         const int b = (int)(t / n);
-        const long long cell = t - (long long)b * n;
-        const int j = (int)(cell / nx), i = (int)(cell - (long long)j * nx);
-        auto cx = [&](int v, int ii, int jj) {  // x-face correction on the left of cell (ii, jj)
-            ii = wrap(ii, nx);
-            jj = wrap(jj, ny);
-            return (double)corr[((long long)(b * 2 + 0) * 4 + v) * n + (long long)jj * nx + ii];
-        };
-        auto cy = [&](int v, int ii, int jj) {
-            ii = wrap(ii, nx);
-            jj = wrap(jj, ny);
-            return (double)corr[((long long)(b * 2 + 1) * 4 + v) * n + (long long)jj * nx + ii];
-        };
-        auto err = [&](int v, int ii, int jj) {
-            const int i2 = wrap(ii, nx), j2 = wrap(jj, ny);
-            const double div = (cx(v, ii + 1, jj) - cx(v, ii, jj)) * inv_dx + (cy(v, ii, jj + 1) - cy(v, ii, jj)) * inv_dy;
-            return resid[((long long)b * 4 + v) * n + (long long)j2 * nx + i2] + div;
-        };
+        const int cell = (int)(t - (long long)b * n);
+        const int j = cell / nx, i = cell - j * nx;
+        const int im = i == 0 ? nx - 1 : i - 1, ip = i == nx - 1 ? 0 : i + 1;
+        const int jr = j * nx, jm = (j == 0 ? ny - 1 : j - 1) * nx, jp = (j == ny - 1 ? 0 : j + 1) * nx;
         const float w[4] = {w0, w1, w2, w3};
         const double scale = 2.0 / (double)total;
+#pragma unroll
         for (int v = 0; v < 4; ++v) {
-            const double e = err(v, i, j);
+            const float* cx = corr + ((long long)(b * 2 + 0) * 4 + v) * n;  // x face on the left of a cell
+            const float* cy = corr + ((long long)(b * 2 + 1) * 4 + v) * n;  // y face below it
+            const double* rs = resid + ((long long)b * 4 + v) * n;
+            const double x0 = cx[jr + i], y0 = cy[jr + i];
+            auto err = [&](double r, double xr, double xl, double yt, double yb) {
+                return r + ((xr - xl) * inv_dx + (yt - yb) * inv_dy);
+            };
+            const double e = err(rs[jr + i], cx[jr + ip], x0, cy[jp + i], y0);
+            const double ex = err(rs[jr + im], x0, cx[jr + im], cy[jp + im], cy[jr + im]);
+            const double ey = err(rs[jm + i], cx[jm + ip], cx[jm + i], y0, cy[jm + i]);
             l += w[v] * e * e;
             // x face on the left of (i, j): +1/dx in cell (i-1, j), -1/dx in cell (i, j)
-            const double gx = scale * w[v] * (err(v, i - 1, j) - e) * inv_dx;
-            const double gy = scale * w[v] * (err(v, i, j - 1) - e) * inv_dy;
-            dcorr[((long long)(b * 2 + 0) * 4 + v) * n + cell] = (float)gx;
-            dcorr[((long long)(b * 2 + 1) * 4 + v) * n + cell] = (float)gy;
+            dcorr[((long long)(b * 2 + 0) * 4 + v) * n + cell] = (float)(scale * w[v] * (ex - e) * inv_dx);
+            dcorr[((long long)(b * 2 + 1) * 4 + v) * n + cell] = (float)(scale * w[v] * (ey - e) * inv_dy);
         }
     }
     for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-    if ((threadIdx.x & 31) == 0 && l != 0.0) atomicAdd(loss, l / (double)total);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = l;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int k = 1; k < 8; ++k) l += red[k];
+        if (l != 0.0) atomicAdd(loss, l / (double)total);
+    }
 }
 
 // Adam on the FP32 parameters, then the BF16 copies the tensor cores read.
@@ -629,21 +672,52 @@ nn::Net nn_net(const efvm_nn* h) {
     return n;
 }
 
+template <typename... KArgs, typename... Args>
+static void launch_nn(void (*kernel)(KArgs...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, bool pdl,
+                      Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+// One persistent block per resident slot, at most one per tile.
+static int nn_blocks(int tiles, int per_sm) {
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return std::min(tiles, per_sm * sms);
+}
+
+static void launch_forward(const nn::PrimView& pv, const efvm_nn* h, int tiles, float* corr, float sensor,
+                           unsigned long long* fallbacks, bool pdl, cudaStream_t s) {
+    launch_nn(nn::nn_forward_kernel, (unsigned)nn_blocks(tiles, nn::FWD_BLOCKS), 128u, (size_t)nn::SM_FWD, s, pdl, pv,
+              nn_net(h), tiles, corr, sensor, fallbacks);
+}
+
+// Both launches belong to a captured step: programmatic, like its other kernels
+// (the weights do not change while a step runs).
 int nn_forward_padded(const efvm_nn* h, const double* q, long long plane, int pitch, int nx, int ny, float* corr,
                       float4* prims, float sensor, unsigned long long* fallbacks, void* stream) {
     cudaStream_t s = (cudaStream_t)stream;
     nn::PaddedState sv{q, plane, pitch, nx, ny};
-    nn::nn_prims_kernel<nn::PaddedState><<<(nx * ny + 255) / 256, 256, 0, s>>>(sv, 1, h->gamma, prims);
-    const int tiles = (int)(2LL * nx * ny / 128);
-    nn::nn_forward_kernel<<<tiles, 128, nn::SM_FWD, s>>>(nn::PrimView{prims, nx, ny}, nn_net(h), corr, sensor,
-                                                          fallbacks);
+    launch_nn(nn::nn_prims_kernel<nn::PaddedState>, (unsigned)((nx * ny + 255) / 256), 256u, (size_t)0, s, true, sv, 1,
+              h->gamma, prims);
+    launch_forward(nn::PrimView{prims, nx, ny}, h, (int)(2LL * nx * ny / 128), corr, sensor, fallbacks, true, s);
     return 2;
 }
 
 int nn_prepare_launches() {
     cudaError_t e = cudaFuncSetAttribute(nn::nn_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, nn::SM_FWD);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(nn::nn_backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, nn::SM_TOTAL);
+        e = cudaFuncSetAttribute(nn::nn_backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, nn::SM_BWD);
     return e == cudaSuccess ? EFVM_OK : EFVM_ERR_CUDA;
 }
 }  // namespace efvm
@@ -694,13 +768,14 @@ int check_shape(efvm_nn* h, int batch, int nx, int ny) {
 }
 
 int ensure_buffers(efvm_nn* h, int batch, int nx, int ny) {
-    const size_t faces = 2ull * batch * nx * ny, tiles = faces / 128;
-    if (tiles * nn::P_COUNT > h->partials_cap) {
+    const size_t faces = 2ull * batch * nx * ny;
+    const size_t blocks = (size_t)nn_blocks((int)(faces / 128), nn::BWD_BLOCKS);
+    if (blocks * nn::P_COUNT > h->partials_cap) {
         cudaFree(h->partials);
         h->partials = nullptr;
         h->partials_cap = 0;
-        NN_TRY(h, cudaMalloc(&h->partials, tiles * nn::P_COUNT * sizeof(float)));
-        h->partials_cap = tiles * nn::P_COUNT;
+        NN_TRY(h, cudaMalloc(&h->partials, blocks * nn::P_COUNT * sizeof(float)));
+        h->partials_cap = blocks * nn::P_COUNT;
     }
     if ((size_t)batch * nx * ny > h->prims_cap) {
         cudaFree(h->prims);
@@ -751,7 +826,7 @@ int efvm_nn_create(float out_scale, float gamma, uint64_t seed, efvm_nn** out) {
     const size_t pb = nn::P_COUNT * sizeof(float);
     if (cudaMalloc(&h->p, pb) || cudaMalloc(&h->m, pb) || cudaMalloc(&h->v, pb) || cudaMalloc(&h->grad, pb) ||
         cudaMalloc(&h->w1, nn::H * nn::K1 * 2) || cudaMalloc(&h->w2, nn::H * nn::H * 2) ||
-        cudaMalloc(&h->w3, nn::N3 * nn::H * 2) || cudaMalloc(&h->loss_d, sizeof(double)))
+        cudaMalloc(&h->w3, nn::N3 * nn::H * 2) || cudaMalloc(&h->loss_d, 2 * sizeof(double)))
         return bad(nfail(nullptr, EFVM_ERR_OOM, "efvm_nn_create: cudaMalloc"));
     cudaMemset(h->m, 0, pb);
     cudaMemset(h->v, 0, pb);
@@ -817,7 +892,7 @@ int efvm_nn_forward(efvm_nn* h, const double* states, int32_t batch, int32_t nx,
     const long long cells = (long long)batch * nx * ny;
     nn::nn_prims_kernel<nn::PackedStates><<<(unsigned)((cells + 255) / 256), 256, 0, s>>>(sv, batch, h->gamma, h->prims);
     const int tiles = (int)(2LL * batch * nx * ny / 128);
-    nn::nn_forward_kernel<<<tiles, 128, nn::SM_FWD, s>>>(nn::PrimView{h->prims, nx, ny}, nn_net(h), corr, 0.f, nullptr);
+    launch_forward(nn::PrimView{h->prims, nx, ny}, h, tiles, corr, 0.f, nullptr, false, s);
     NN_TRY(h, cudaGetLastError());
     NN_TRY(h, cudaStreamSynchronize(s));
     return tc_status(h);
@@ -836,18 +911,21 @@ int efvm_nn_loss_grad(efvm_nn* h, const double* states, const double* resid, int
     const int tiles = (int)(2 * cells / 128);
     nn::nn_prims_kernel<nn::PackedStates><<<(unsigned)((cells + 255) / 256), 256, 0, s>>>(sv, batch, h->gamma, h->prims);
     const nn::PrimView pv{h->prims, nx, ny};
-    nn::nn_forward_kernel<<<tiles, 128, nn::SM_FWD, s>>>(pv, nn_net(h), h->corr, 0.f, nullptr);
+    launch_forward(pv, h, tiles, h->corr, 0.f, nullptr, false, s);
     NN_TRY(h, cudaMemsetAsync(h->loss_d, 0, sizeof(double), s));
     nn::nn_residual_kernel<<<(unsigned)((cells + 255) / 256), 256, 0, s>>>(h->corr, resid, batch, nx, ny, 1.0 / dx,
                                                                          1.0 / dy, w[0], w[1], w[2], w[3], h->dcorr,
                                                                          h->loss_d);
-    nn::nn_backward_kernel<<<tiles, 128, nn::SM_TOTAL, s>>>(pv, nn_net(h), h->dcorr, h->partials);
-    nn::nn_reduce_kernel<<<(nn::P_COUNT + 255) / 256, 256, 0, s>>>(h->partials, tiles, h->grad);
-    if (grad_out) NN_TRY(h, cudaMemcpyAsync(grad_out, h->grad, nn::P_COUNT * sizeof(float), cudaMemcpyDeviceToDevice, s));
+    const int blocks = nn_blocks(tiles, nn::BWD_BLOCKS);
+    nn::nn_backward_kernel<<<blocks, 128, nn::SM_BWD, s>>>(pv, nn_net(h), tiles, h->dcorr, h->partials);
+    nn::nn_reduce_kernel<<<(nn::P_COUNT + 31) / 32, 32 * nn::RED_SLICES, 0, s>>>(h->partials, blocks, h->grad, grad_out,
+                                                                                 h->loss_d);
     NN_TRY(h, cudaGetLastError());
-    if (loss) NN_TRY(h, cudaMemcpyAsync(loss, h->loss_d, sizeof(double), cudaMemcpyDeviceToHost, s));
+    double out[2] = {0.0, 0.0};  // the loss and the tensor-core status
+    NN_TRY(h, cudaMemcpyAsync(out, h->loss_d, sizeof(out), cudaMemcpyDeviceToHost, s));
     NN_TRY(h, cudaStreamSynchronize(s));
-    return tc_status(h);
+    if (loss) *loss = out[0];
+    return out[1] != 0.0 ? tc_status(h) : EFVM_OK;
 }
 
 int efvm_nn_adam(efvm_nn* h, float lr, void* stream) {

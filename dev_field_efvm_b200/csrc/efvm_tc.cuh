@@ -13,6 +13,12 @@
 // 2 s LBO.  The accumulator D (M = 128 rows) occupies TMEM lane r, column j
 // for element (r, j), 32 bits each.
 //
+// The same bytes read the other way round are the canonical MN-major layout of
+// the transpose: the 16 contiguous bytes run along M (or N), the 8 rows of a
+// core matrix along K, core matrices adjacent in M are SBO = 16 R bytes apart
+// and those adjacent in K LBO = 128 bytes.  An operand stored once therefore
+// serves a product and the product with its transpose.
+//
 // Every wait is bounded: a wait that runs out records an error code and the
 // kernel carries on to its clean-up (TMEM is always released).
 #pragma once
@@ -53,6 +59,9 @@ __host__ __device__ constexpr uint32_t idesc_bf16_f32(int m, int n) {
            | ((uint32_t)(n >> 3) << 17)    // N >> 3
            | ((uint32_t)(m >> 4) << 24);   // M >> 4
 }
+
+// The same with A and / or B in the MN-major layout (bits 15 and 16).
+constexpr uint32_t A_MN = 1u << 15, B_MN = 1u << 16;
 
 // ---- tensor memory -------------------------------------------------------
 // Allocation and release by one whole warp; the TMEM address lands in *slot.
@@ -123,6 +132,17 @@ __device__ __forceinline__ void gemm_issue(uint32_t tmem_d, const void* a, const
         }
         mma_commit(bar);
     }
+}
+
+// The same product for operands in either layout, by the calling thread, not
+// committed.  Descriptors advance by step_a / step_b bytes per K = 16.
+__device__ __forceinline__ void mma_steps(uint32_t tmem_d, const void* a, uint32_t lbo_a, uint32_t sbo_a,
+                                          uint32_t step_a, const void* b, uint32_t lbo_b, uint32_t sbo_b,
+                                          uint32_t step_b, uint32_t idesc, int steps, bool accumulate) {
+    const uint32_t sa = smem_u32(a), sb = smem_u32(b);
+    for (int s = 0; s < steps; ++s)
+        mma_bf16(tmem_d, smem_desc(sa + (uint32_t)s * step_a, lbo_a, sbo_a),
+                 smem_desc(sb + (uint32_t)s * step_b, lbo_b, sbo_b), idesc, accumulate || s > 0);
 }
 
 // ---- accumulator read-back -------------------------------------------------
