@@ -12,13 +12,14 @@ import os
 import shutil
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libefvm_b200.so")
 BUILD = os.path.join(HERE, "_build")
-SOURCES = ["efvm_kernels.cu", "efvm_api.cu", "efvm_batch.cu", "efvm_nn.cu", "efvm_noalloc.cu"]
-HEADERS = ["efvm_internal.h", "efvm_math.cuh", "efvm_kernels3d.cuh", "efvm_tc.cuh", "efvm_tma.cuh", "../../include/efvm.h"]
+SOURCES = ["efvm_kernels.cu", "efvm_tile.cu", "efvm_api.cu", "efvm_batch.cu", "efvm_nn.cu", "efvm_noalloc.cu"]
+HEADERS = ["efvm_internal.h", "efvm_math.cuh", "efvm_device.cuh", "efvm_kernels3d.cuh", "efvm_tc.cuh", "efvm_tma.cuh", "../../include/efvm.h"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -47,16 +48,18 @@ def build(verbose: bool = False, force: bool = False) -> str:
     if not force and _newer(OUT, deps):
         return OUT
     os.makedirs(BUILD, exist_ok=True)
-    objs = []
-    log = []
-    for src in SOURCES:
-        obj = os.path.join(BUILD, src.replace(".cu", ".o"))
+    objs = [os.path.join(BUILD, src.replace(".cu", ".o")) for src in SOURCES]
+
+    def compile_one(src, obj):
         cmd = [nvcc(), *NVCC_FLAGS, "-c", os.path.join(CSRC, src), "-o", obj]
-        r = subprocess.run(cmd, capture_output=True, text=True)
-        log.append(r.stdout + r.stderr)
+        return subprocess.run(cmd, capture_output=True, text=True)
+
+    with ThreadPoolExecutor() as pool:  # the files are independent
+        done = list(pool.map(compile_one, SOURCES, objs))
+    log = [r.stdout + r.stderr for r in done]
+    for src, r in zip(SOURCES, done):
         if r.returncode != 0:
             raise RuntimeError(f"nvcc failed for {src}:\n{r.stderr}")
-        objs.append(obj)
     tmp = OUT + ".tmp"
     cmd = [nvcc(), "-gencode", "arch=compute_100a,code=sm_100a", "-shared", "-cudart", "static",
            "-Xcompiler", "-fPIC", *objs, "-o", tmp]

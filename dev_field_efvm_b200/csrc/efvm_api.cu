@@ -525,6 +525,16 @@ int resolved_form(const efvm_ctx* c) {
     return EFVM_STAGE_STRIP;
 }
 
+// Whether the built-in choice is the face-parallel kernel (efvm_tile.cu): an FP64
+// case of at most TILE_CELLS cells whose form and rows are not set explicitly.
+// The line lies where the two forms measured equal (efvm_tile.cu): the TMA-fed
+// form overtakes it near 1024^2, the viscous strip form near 2200x410.
+constexpr long long TILE_CELLS = 800000;
+bool use_tile(const efvm_ctx* c) {
+    return c->g.nz <= 1 && c->ph.precision == EFVM_PREC_FP64 && c->stage_form == EFVM_STAGE_AUTO &&
+           c->stage_rows == 0 && c->stage_blocks == 0 && (long long)c->g.nx * c->g.ny <= TILE_CELLS;
+}
+
 void enqueue_stage_kernel(efvm_ctx* c, int stage, double* uin, double* uout, bool pdl = true, bool defer = false) {
     if (c->nn)  // the learned corrections of this stage's input
         c->launches += nn_forward_padded(c->nn, uin, c->g.plane, c->g.pitch, c->g.nx, c->g.ny, c->corr, c->prims,
@@ -549,6 +559,7 @@ void enqueue_stage_kernel(efvm_ctx* c, int stage, double* uin, double* uout, boo
             if (uin == c->U[k]) a.tmap_in = &c->tmap[k];
         a.tmap_u0 = &c->tmap_u0;
     }
+    a.tile = use_tile(c);
     a.rows = c->stage_rows;
     a.blocks = c->stage_blocks;
     a.wait_ns = c->stage_wait_ns;
@@ -1791,6 +1802,12 @@ static int resolved_blocks(const efvm_ctx* c, int form) {
 
 int efvm_get_stage_tiling(efvm_ctx* c, int32_t* form, int32_t* rows_per_warp, int32_t* blocks_per_sm) {
     if (!c || !form || !rows_per_warp || !blocks_per_sm) return fail(c, EFVM_ERR_INVALID_ARG, "null argument");
+    if (use_tile(c)) {  // the face-parallel build counts as the strip form's
+        *form = EFVM_STAGE_STRIP;
+        *rows_per_warp = TILE_ROWS;
+        *blocks_per_sm = resolved_blocks(c, EFVM_STAGE_STRIP);
+        return EFVM_OK;
+    }
     *form = resolved_form(c);
     *blocks_per_sm = resolved_blocks(c, *form);
     *rows_per_warp = c->stage_rows > 0 ? c->stage_rows
@@ -1809,7 +1826,7 @@ int efvm_get_stage_tiling(efvm_ctx* c, int32_t* form, int32_t* rows_per_warp, in
 // fastest: the strip kernel at its built-in and its alternate resident-block
 // count and (where the case allows it) the TMA-fed kernel, each with 4, 8, 16
 // and 32 rows per warp and with the rows that fit the whole grid into one wave
-// of resident blocks.  The state, the clock and the force
+// of resident blocks, and the face-parallel kernel where it is the built-in choice.  The state, the clock and the force
 // outputs are saved first and restored after every candidate, so tuning
 // changes no result.
 int efvm_autotune_stage(efvm_ctx* c, int32_t n_steps, double* best_ms_per_step) {
@@ -1857,6 +1874,9 @@ int efvm_autotune_stage(efvm_ctx* c, int32_t n_steps, double* best_ms_per_step) 
     if (alt > 0) shapes.push_back({EFVM_STAGE_STRIP, alt});
     for (int form : forms)
         if (form == EFVM_STAGE_TMA) shapes.push_back({EFVM_STAGE_TMA, 0});
+    c->stage_form = EFVM_STAGE_AUTO;
+    c->stage_rows = c->stage_blocks = 0;
+    if (use_tile(c)) shapes.push_back({EFVM_STAGE_AUTO, 0});  // the built-in choice, one shape
     for (const auto& shape : shapes) {
         const int form = shape.first, blocks = shape.second;
         // one wave: the rows that spread the grid's strips over every resident block once
@@ -1866,6 +1886,7 @@ int efvm_autotune_stage(efvm_ctx* c, int32_t n_steps, double* best_ms_per_step) 
         std::vector<int> rows{4, 8, 16, 32, (c->g.ny + by - 1) / by};
         std::sort(rows.begin(), rows.end());
         rows.erase(std::unique(rows.begin(), rows.end()), rows.end());
+        if (form == EFVM_STAGE_AUTO) rows.assign(1, 0);
         for (int r : rows) {
             if (r > c->g.ny && r != rows.front()) continue;
             c->stage_form = form;

@@ -207,6 +207,7 @@ struct StageArgs {
     const void* tmap_in;
     const void* tmap_u0;
     int rows;                         // rows per warp; 0 = the built-in choice
+    int tile;                         // 1: the face-parallel kernel (efvm_tile.cu)
     int blocks;                       // resident blocks per SM of the strip form; 0 = the built-in choice
     unsigned long long wait_ns;       // limit of one wait of the TMA-fed kernel for a row (ns)
     int stall;                        // failure injection: the first block's ring stops being refilled
@@ -281,6 +282,10 @@ int stage_alt_blocks(bool fp32, bool viscous);
 // box of the stage input (u0 = false) or of U^n (u0 = true); 0 on success.
 bool stage_tma_eligible(const Geometry& g, const Physics& ph, bool ibm, bool corr);
 int encode_state_map(const Geometry& g, const double* buf, bool u0, void* map_out);
+// The face-parallel stage kernel (efvm_tile.cu): 2-D FP64 cases, tiles of
+// 31 columns x TILE_ROWS rows, TILE_BLOCKS resident blocks per SM.
+constexpr int TILE_ROWS = 3, TILE_BLOCKS = 4;
+int launch_stage_tile(const StageArgs& a, bool pdl, void* stream);
 int launch_batch_stage(const BatchStageArgs& b, int n_tiles, bool pdl, void* stream);
 // Per-step set-up of every case (one thread each).
 int launch_batch_setup(const Physics& ph, const BatchCase* cases, int n_cases, bool pdl, void* stream);

@@ -104,6 +104,126 @@ __device__ __forceinline__ Q4<R> physical_flux(R rho, R un, R ut, R E, R p) {
     return f;
 }
 
+// ---- FP64 fluxes ------------------------------------------------------------
+// Every operation of the FP64 fluxes is rounded explicitly (the compiler neither
+// fuses nor splits them), so a face formed by different kernels, or by two
+// warps of one, has the same bits whatever code surrounds it.
+struct SideD {
+    double un, ut, q, p, a2, a;
+};
+__device__ __forceinline__ SideD side_d(const Q4<double>& u, double inv, double gamma, double gm1) {
+    SideD s;
+    s.un = __dmul_rn(u.mn, inv);
+    s.ut = __dmul_rn(u.mt, inv);
+    s.q = __fma_rn(s.un, s.un, __dmul_rn(s.ut, s.ut));
+    s.p = __dmul_rn(gm1, __fma_rn(__dmul_rn(-0.5, u.r), s.q, u.E));
+    s.a2 = __dmul_rn(__dmul_rn(gamma, s.p), inv);
+    s.a = __dmul_rn(s.a2, rsqrt_(s.a2));  // NaN for a non-physical p <= 0, which the stage flags
+    return s;
+}
+__device__ __forceinline__ void sides_d(const Q4<double>& L, const Q4<double>& R, double gamma, double gm1, SideD& l,
+                                        SideD& r) {
+    const double w = rcp_(__dmul_rn(L.r, R.r));
+    l = side_d(L, __dmul_rn(R.r, w), gamma, gm1);
+    r = side_d(R, __dmul_rn(L.r, w), gamma, gm1);
+}
+// physical_flux_inline, crates/cfd_riemann/src/lib.rs:21-43
+__device__ __forceinline__ Q4<double> physical_flux_d(double rho, double un, double ut, double E, double p) {
+    Q4<double> f;
+    f.r = __dmul_rn(rho, un);
+    f.mn = __fma_rn(f.r, un, p);
+    f.mt = __dmul_rn(f.r, ut);
+    f.E = __dmul_rn(__dadd_rn(E, p), un);
+    return f;
+}
+// Rusanov::flux_inline, crates/cfd_riemann/src/lib.rs:222-240
+__device__ __forceinline__ Q4<double> rusanov_flux_d(const Q4<double>& L, const Q4<double>& R, double gamma,
+                                                     double gm1) {
+    SideD l, r;
+    sides_d(L, R, gamma, gm1, l, r);
+    const Q4<double> fl = physical_flux_d(L.r, l.un, l.ut, L.E, l.p);
+    const Q4<double> fr = physical_flux_d(R.r, r.un, r.ut, R.E, r.p);
+    const double hl = __dmul_rn(-0.5, fmax(__dadd_rn(fabs(l.un), l.a), __dadd_rn(fabs(r.un), r.a)));
+    auto mix = [&](double a, double b, double ul, double ur) {
+        return __fma_rn(hl, __dsub_rn(ur, ul), __dmul_rn(0.5, __dadd_rn(a, b)));
+    };
+    return Q4<double>{mix(fl.r, fr.r, L.r, R.r), mix(fl.mn, fr.mn, L.mn, R.mn), mix(fl.mt, fr.mt, L.mt, R.mt),
+                      mix(fl.E, fr.E, L.E, R.E)};
+}
+// Hllc::flux_with_thornber + thornber_reconstruct + star_state,
+// crates/cfd_riemann/src/lib.rs:395-506,619-644, in an equivalent form:
+//  * the Thornber blend keeps rho and the internal energy, hence p and a (the
+//    reference's cached path relies on the same identity, :586-588), and the
+//    blended velocities are used directly;
+//  * the upwind side K (left for s_l >= 0 or s_* >= 0, else right) is selected
+//    first.  In the star regions the flux is the star state's physical flux,
+//    which equals F_K + s_K (U*_K - U_K): with f_K = rho_K (s_K - u_K),
+//    rho* = f_K / (s_K - s_*), m = rho* s_*, p* = p_K + f_K (s_* - u_K),
+//    E* = ((s_K - u_K) E_K - p_K u_K + p* s_*) / (s_K - s_*),
+//    F = (m, m s_* + p*, m t_K, (E* + p*) s_*);
+//  * s_* = n/d and 1/(s_K - s_*) = d/(s_K d - n) come from one reciprocal of
+//    d (s_K d - n), and only in the star regions: elsewhere the sign of s_* is
+//    read from the sign of n d;
+//  * a_max^2 is the larger a^2, a side without a positive one left out (as the
+//    maximum of the sound speeds leaves out a NaN).
+template <bool THORNBER>
+__device__ __forceinline__ Q4<double> hllc_flux_d(const Q4<double>& L, const Q4<double>& R, double gamma, double gm1) {
+    SideD l, r;
+    sides_d(L, R, gamma, gm1, l, r);
+    double lcn = l.un, lct = l.ut, rcn = r.un, rct = r.ut, ELc = L.E, ERc = R.E;
+    if (THORNBER) {
+        // z = min(|v|max / a_max, 1) as vmax2 / sqrt(vmax2 a_max^2): one reciprocal square
+        // root.  Where vmax2 a_max^2 is below the normal range (round-off velocities
+        // near 1e-157 in still gas), z is taken as 0: the reference's z there is
+        // about 1e-160 and scales velocity differences of the same size, far below
+        // any representable change of the flux.
+        const double vmax2 = l.q > r.q ? l.q : r.q;
+        const double amax2 = l.a2 > r.a2 ? l.a2 : r.a2;
+        const double prod = __dmul_rn(vmax2, amax2);
+        double hz = __dmul_rn(__dmul_rn(0.5, vmax2), rsqrt_(prod));
+        hz = prod >= normal_min<double>() ? hz : 0.0;
+        hz = vmax2 >= amax2 && amax2 > 0.0 ? 0.5 : hz;
+        const double avgn = __dmul_rn(0.5, __dadd_rn(l.un, r.un)), avgt = __dmul_rn(0.5, __dadd_rn(l.ut, r.ut));
+        const double dun = __dsub_rn(l.un, r.un), dut = __dsub_rn(l.ut, r.ut);
+        lcn = __fma_rn(hz, dun, avgn);
+        lct = __fma_rn(hz, dut, avgt);
+        rcn = __fma_rn(-hz, dun, avgn);
+        rct = __fma_rn(-hz, dut, avgt);
+        ELc = __fma_rn(__dmul_rn(0.5, L.r), __fma_rn(lcn, lcn, __fma_rn(lct, lct, -l.q)), L.E);
+        ERc = __fma_rn(__dmul_rn(0.5, R.r), __fma_rn(rcn, rcn, __fma_rn(rct, rct, -r.q)), R.E);
+    }
+    const double s_l = fmin(__dsub_rn(lcn, l.a), __dsub_rn(rcn, r.a));
+    const double s_r = fmax(__dadd_rn(lcn, l.a), __dadd_rn(rcn, r.a));
+    const double fac_l = __dmul_rn(L.r, __dsub_rn(s_l, lcn));
+    const double fac_r = __dmul_rn(R.r, __dsub_rn(s_r, rcn));
+    const double num = __fma_rn(-fac_r, rcn, __fma_rn(fac_l, lcn, __dsub_rn(r.p, l.p)));
+    const double den = __dsub_rn(fac_l, fac_r);
+    // s_* = num / den >= 0 without the division (false for den = 0 or NaN)
+    const bool star_nonneg = __dmul_rn(num, den) >= 0.0 && den != 0.0;
+    const bool useL = (s_l >= 0.0) || star_nonneg;
+    const double uK = useL ? lcn : rcn;
+    const double tK = useL ? lct : rct;
+    const double EK = useL ? ELc : ERc;
+    const double pK = useL ? l.p : r.p;
+    if (s_l < 0.0 && (star_nonneg || s_r >= 0.0)) {  // one of the two star regions
+        const double sK = useL ? s_l : s_r;
+        const double facK = useL ? fac_l : fac_r;
+        const double Y = __fma_rn(sK, den, -num);
+        const double w = rcp_(__dmul_rn(den, Y));
+        const double s_star = __dmul_rn(num, __dmul_rn(Y, w));
+        const double inv = __dmul_rn(den, __dmul_rn(den, w));  // 1 / (s_K - s_*)
+        const double pS = __fma_rn(facK, __dsub_rn(s_star, uK), pK);
+        Q4<double> f;
+        f.r = __dmul_rn(__dmul_rn(facK, inv), s_star);
+        f.mn = __fma_rn(f.r, s_star, pS);
+        f.mt = __dmul_rn(f.r, tK);
+        const double eS = __fma_rn(pS, s_star, __fma_rn(__dsub_rn(sK, uK), EK, -__dmul_rn(pK, uK)));
+        f.E = __dmul_rn(__fma_rn(eS, inv, pS), s_star);
+        return f;
+    }
+    return physical_flux_d(useL ? L.r : R.r, uK, tK, EK, pK);
+}
+
 // Rusanov::flux_inline, crates/cfd_riemann/src/lib.rs:222-240
 template <class R>
 __device__ __forceinline__ Q4<R> rusanov_flux(const Q4<R>& L, const Q4<R>& Rr, R gamma, R gm1) {
@@ -201,9 +321,13 @@ __device__ __forceinline__ Q4<R> hllc_flux(const Q4<R>& L, const Q4<R>& Rr, R ga
 
 template <int SCHEME, class R>
 __device__ __forceinline__ Q4<R> face_flux(const Q4<R>& L, const Q4<R>& Rr, R gamma, R gm1) {
-    if (SCHEME == EFVM_FLUX_RUSANOV) return rusanov_flux(L, Rr, gamma, gm1);
-    if (SCHEME == EFVM_FLUX_HLLC_TEXTBOOK) return hllc_flux<R, false>(L, Rr, gamma, gm1);
-    return hllc_flux<R, true>(L, Rr, gamma, gm1);
+    if constexpr (sizeof(R) == sizeof(double)) {
+        if (SCHEME == EFVM_FLUX_RUSANOV) return rusanov_flux_d(L, Rr, gamma, gm1);
+        return hllc_flux_d<SCHEME != EFVM_FLUX_HLLC_TEXTBOOK>(L, Rr, gamma, gm1);
+    } else {
+        if (SCHEME == EFVM_FLUX_RUSANOV) return rusanov_flux(L, Rr, gamma, gm1);
+        return hllc_flux<R, SCHEME != EFVM_FLUX_HLLC_TEXTBOOK>(L, Rr, gamma, gm1);
+    }
 }
 
 // ---- 3-D: states (rho, m_n, m_t, m_s, E) in the frame of the face normal,
@@ -355,6 +479,26 @@ __device__ __forceinline__ R monotonized_central(R a, R b) {
 template <class R>
 __device__ __forceinline__ R limit(int limiter, R fwd, R bwd) {
     return limiter == EFVM_LIMITER_MC ? monotonized_central(fwd, bwd) : minmod(fwd, bwd);
+}
+
+// The limited slope for the FP64 forms that apply it as c +- s f: s is the
+// limiter's value as if the differences had the same sign, and f is `factor` (0.5,
+// or 0 on a first-order side) or 0 where they have opposite signs.  The sign
+// test is one bit operation on the high words instead of a product and a
+// comparison, and the zero of the limiter costs one select of f's high word (the
+// low word of 0.5 and 0 is zero) instead of two of s.  The states have the bits
+// of c +- limit() / 2, except where a difference product underflows (|a b| <
+// 1e-308), whose slope is kept instead of dropped.
+__device__ __forceinline__ void limited_slope(int limiter, double fwd, double bwd, double factor, double& s, double& f) {
+    const bool opposite = (__double2hiint(fwd) ^ __double2hiint(bwd)) < 0;
+    f = __hiloint2double(opposite ? 0 : __double2hiint(factor), 0);
+    if (limiter == EFVM_LIMITER_MC) {
+        const double a = fabs(fwd), b = fabs(bwd), h = __dmul_rn(0.5, fabs(__dadd_rn(fwd, bwd)));
+        const double m = __dmul_rn(2.0, a < b ? a : b);
+        s = copysign(m < h ? m : h, fwd);
+    } else {
+        s = fabs(fwd) < fabs(bwd) ? fwd : bwd;
+    }
 }
 
 }  // namespace efvm
