@@ -1816,8 +1816,7 @@ int efvm_get_stage_tiling(efvm_ctx* c, int32_t* form, int32_t* rows_per_warp, in
     if (c->stage_rows <= 0 && *blocks_per_sm != stage_blocks_per_sm(c->ph.precision == EFVM_PREC_FP32_FLUX,
                                                                      c->ph.viscous != 0, *form == EFVM_STAGE_TMA)) {
         // the built-in rows follow the resident slots of the count in use
-        const long long strips = stage_strips(c->g.nx), slots = 148LL * *blocks_per_sm * 4;
-        *rows_per_warp = (int)std::min<long long>(16, std::max<long long>(2, (strips * c->g.ny + slots - 1) / slots));
+        *rows_per_warp = stage_rows_for(c->g.nx, c->g.ny, *blocks_per_sm);
     }
     return EFVM_OK;
 }

@@ -272,6 +272,7 @@ int batch_form_blocks(bool fp32, bool viscous);
 // case that runs alone (fp32: the FP32-flux form; viscous: with viscous terms).
 int stage_strips(int nx);
 int stage_rows(int nx, int ny, bool fp32, bool viscous, bool tma = false);
+int stage_rows_for(int nx, int ny, int blocks_per_sm);
 // Resident blocks per SM of the stage-kernel form (tma: the TMA-fed kernel), and
 // the strip form's second choice for the autotuner (0: none).
 int stage_blocks_per_sm(bool fp32, bool viscous, bool tma);

@@ -8,9 +8,12 @@
 // (i, j, k) sits at layer ZO + k, row YO + j, column XO + i.  Layers ZO-2,
 // ZO-1 and ZO+nz, ZO+nz+1 are the two z ghost layers of FIELD's ng = 2.
 //
-// The stage kernel keeps the 2-D kernel's organisation: a warp owns a strip of
-// 31 columns of one layer k and marches `rows` rows with the carried y window,
-// and the x faces come from warp shuffles.  The warps of a block stack in z
+// The stage kernel keeps the 2-D strip kernel's organisation: a warp owns a strip
+// of 31 or 32 columns of one layer k and marches `rows` rows with the carried y
+// window; each lane forms the x face on the left of its column from the four
+// cells about it.  With 31 columns lane 31 forms the last right face in every
+// row, with 32 it comes from one pass over the rows, a row per lane, before the
+// march: that pays where it saves a strip (128 columns: 4 instead of 5).  The warps of a block stack in z
 // over the same strip and rows and share the z direction through shared
 // memory: each limits the z slope of its own cell once and forms the z face
 // above its layer once.  A z face on the edge of two blocks is formed by both
@@ -142,22 +145,22 @@ struct V5 {
 };
 __device__ __forceinline__ V5 toV5(const U5& u) { return V5{u.r, u.mx, u.my, u.mz, u.E}; }
 __device__ __forceinline__ U5 toU5(const V5& u) { return U5{u.r, u.mx, u.my, u.mz, u.E}; }
-__device__ __forceinline__ Q5<double> xq5(const V5& u) { return Q5<double>{u.r, u.mx, u.my, u.mz, u.E}; }
-__device__ __forceinline__ Q5<double> yq5(const V5& u) { return Q5<double>{u.r, u.my, u.mx, u.mz, u.E}; }
-__device__ __forceinline__ Q5<double> zq5(const V5& u) { return Q5<double>{u.r, u.mz, u.mx, u.my, u.E}; }
+__device__ __forceinline__ Q5 xq5(const V5& u) { return Q5{u.r, u.mx, u.my, u.mz, u.E}; }
+__device__ __forceinline__ Q5 yq5(const V5& u) { return Q5{u.r, u.my, u.mx, u.mz, u.E}; }
+__device__ __forceinline__ Q5 zq5(const V5& u) { return Q5{u.r, u.mz, u.mx, u.my, u.E}; }
 // A face flux back in the grid frame (x, y, z faces).
-__device__ __forceinline__ V5 xg5(const Q5<double>& f) { return V5{f.r, f.mn, f.mt, f.ms, f.E}; }
-__device__ __forceinline__ V5 yg5(const Q5<double>& f) { return V5{f.r, f.mt, f.mn, f.ms, f.E}; }
-__device__ __forceinline__ V5 zg5(const Q5<double>& f) { return V5{f.r, f.mt, f.ms, f.mn, f.E}; }
+__device__ __forceinline__ V5 xg5(const Q5& f) { return V5{f.r, f.mn, f.mt, f.ms, f.E}; }
+__device__ __forceinline__ V5 yg5(const Q5& f) { return V5{f.r, f.mt, f.mn, f.ms, f.E}; }
+__device__ __forceinline__ V5 zg5(const Q5& f) { return V5{f.r, f.mt, f.ms, f.mn, f.E}; }
 
 // The +face and -face states c +- s/2 of a cell, s = lim(p - c, c - m)
 // (limited_slope_cons and reconstruct_to_face, crates/cfd_solver/src/lib.rs:199-211,273-286).
 __device__ __forceinline__ void slope_faces5(int limiter, const V5& m, const V5& c, const V5& p, V5& plus, V5& minus) {
-    const double hr = half_slope(limiter, m.r, c.r, p.r), hx = half_slope(limiter, m.mx, c.mx, p.mx);
-    const double hy = half_slope(limiter, m.my, c.my, p.my), hz = half_slope(limiter, m.mz, c.mz, p.mz);
-    const double he = half_slope(limiter, m.E, c.E, p.E);
-    plus = V5{c.r + hr, c.mx + hx, c.my + hy, c.mz + hz, c.E + he};
-    minus = V5{c.r - hr, c.mx - hx, c.my - hy, c.mz - hz, c.E - he};
+    slope_pair(limiter, m.r, c.r, p.r, 0.5, 0.5, plus.r, minus.r);
+    slope_pair(limiter, m.mx, c.mx, p.mx, 0.5, 0.5, plus.mx, minus.mx);
+    slope_pair(limiter, m.my, c.my, p.my, 0.5, 0.5, plus.my, minus.my);
+    slope_pair(limiter, m.mz, c.mz, p.mz, 0.5, 0.5, plus.mz, minus.mz);
+    slope_pair(limiter, m.E, c.E, p.E, 0.5, 0.5, plus.E, minus.E);
 }
 
 __device__ __forceinline__ V5 shfl_up5(const V5& u, int d) {
@@ -181,6 +184,7 @@ __device__ __forceinline__ void prim5(const U5& u, double inv, double gm1, doubl
     t = gm1 * (u.E - ke) * inv * inv_r_gas;
 }
 
+constexpr int ROWS3 = 16;   // most rows it marches
 constexpr int WPB3 = 4;   // warps per block of the 3-D stage kernel, stacked in z
 constexpr int MINB3 = 4;  // resident blocks per SM of the 3-D stage kernel (128 registers)
 
@@ -205,7 +209,7 @@ constexpr int MINB3 = 4;  // resident blocks per SM of the 3-D stage kernel (128
 // LIM >= 0 fixes the limiter and PXYZ a fully periodic mesh at compile time
 // (the inviscid forms are built so); -1 and false read them at run time.
 template <int SCHEME, int RECON, bool VISC, int LIM, bool PXYZ>
-__global__ void __launch_bounds__(32 * WPB3, MINB3) stage3_kernel(StageArgs a, int rows) {
+__global__ void __launch_bounds__(32 * WPB3, MINB3) stage3_kernel(StageArgs a, int rows, int columns) {
     pdl_wait_then_release();
     if (!a.st->active) return;
     const Geometry& g = a.g;
@@ -213,7 +217,8 @@ __global__ void __launch_bounds__(32 * WPB3, MINB3) stage3_kernel(StageArgs a, i
     const int limiter = LIM >= 0 ? LIM : ph.limiter;
     const long long P = g.plane;
     const int lane = threadIdx.x & 31;
-    const int strips = (g.nx + STRIP - 1) / STRIP;
+    const int width = VISC ? 31 : columns;  // the viscous forms have no registers to spare for the edge pass
+    const int strips = (g.nx + width - 1) / width;
     const int warp = threadIdx.x >> 5;
     const int kgroup = blockIdx.x / strips, strip = blockIdx.x - kgroup * strips;
     const int k_raw = kgroup * WPB3 + warp;
@@ -223,6 +228,7 @@ __global__ void __launch_bounds__(32 * WPB3, MINB3) stage3_kernel(StageArgs a, i
     __shared__ double zup[WPB3][5][32];     // the flux of the face above each warp's layer, per lane
     // z face states of the block's column, face f lying below layer WPB3 (b div strips) + f
     __shared__ double zst[2][WPB3 + 1][5][32];  // [left/right state][face][variable][lane]
+    __shared__ double xedge[WPB3][5][ROWS3];    // each warp's flux on the right of its last column, per row
     if (strip == 0 && by == 0 && k_raw == 0 && lane == 0) {
         // RK state machine and clock of update_system, crates/cfd_solver/src/lib.rs:607-621
         DevState* st = a.st;
@@ -237,7 +243,7 @@ __global__ void __launch_bounds__(32 * WPB3, MINB3) stage3_kernel(StageArgs a, i
             st->completed = 0;
         }
     }
-    const int i0 = strip * STRIP;
+    const int i0 = strip * width;
     const int jb = by * rows;
     double lam = 0.0;
     if (jb < g.ny) {  // uniform across the block (its barriers sit inside)
@@ -245,25 +251,47 @@ __global__ void __launch_bounds__(32 * WPB3, MINB3) stage3_kernel(StageArgs a, i
         const int je = min(jb + rows, g.ny);
         const int i = i0 + lane;
         const int ic = min(i, g.nx + NG - 1);
-        const bool owner = lane < STRIP && i < g.nx;
+        const bool owner = lane < width && i < g.nx;
         const bool true_seam = ph.periodic_seam == EFVM_SEAM_TRUE_PERIODIC;
         const double gm1 = ph.gamma - 1.0;
         const double rg = ph.gamma;
         const double* __restrict__ uin = a.uin;
-        auto ld = [&](int ii, int jj, int kk) { return load5(uin, P, cidx3(g, ii, jj, kk)); };
         const double* __restrict__ colp = uin + cidx3(g, ic, 0, k);
         auto ldrow = [&](int jj) { return toV5(load5(colp, P, (long long)jj * g.pitch)); };
         auto ldz = [&](int jj, int dk) { return toV5(load5(colp, P, (long long)jj * g.pitch + (long long)dk * g.layer)); };
 
-        // reconstruction flags of the faces on the domain edges (as the 2-D kernel)
-        bool rec_l = MUSCL, rec_r = MUSCL;
-        if (i == 0) {
-            rec_l = MUSCL && ph.periodic_x && true_seam;
-            rec_r = MUSCL && ph.periodic_x;
-        } else if (i == g.nx) {
-            rec_l = MUSCL && ph.periodic_x;
-            rec_r = MUSCL && ph.periodic_x && true_seam;
-        }
+        // slope factors of the two sides of an x face: 0.5, or 0 on the sides on the
+        // domain edge that take the cell value (as the 2-D kernel)
+        auto x_factors = [&](int f, double& fl, double& fr) {
+            const double in = PXYZ || ph.periodic_x ? 0.5 : 0.0;
+            const double far = (PXYZ || ph.periodic_x) && true_seam ? 0.5 : 0.0;
+            fl = f == 0 ? far : (f == g.nx ? in : 0.5);
+            fr = f == 0 ? in : (f == g.nx ? far : 0.5);
+        };
+        // The x face between the cells at c[-1] and c[0] (c the address of a cell's
+        // density): both slopes from the four cells about it.
+        auto x_flux = [&](const double* __restrict__ c, const V5& left, const V5& right, double fl, double fr) {
+            V5 L = left, R = right;
+            if (MUSCL) {
+                const V5 ll = toV5(load5(c, P, -2)), rr = toV5(load5(c, P, 1));
+                auto side = [&](double q0, double q1, double q2, double q3, double& l, double& r) {
+                    const double d1 = __dsub_rn(q1, q0), d2 = __dsub_rn(q2, q1), d3 = __dsub_rn(q3, q2);
+                    double s, f;
+                    limited_slope(limiter, d2, d1, fl, s, f);
+                    l = __fma_rn(s, f, q1);
+                    limited_slope(limiter, d3, d2, fr, s, f);
+                    r = __fma_rn(-s, f, q2);
+                };
+                side(ll.r, left.r, right.r, rr.r, L.r, R.r);
+                side(ll.mx, left.mx, right.mx, rr.mx, L.mx, R.mx);
+                side(ll.my, left.my, right.my, rr.my, L.my, R.my);
+                side(ll.mz, left.mz, right.mz, rr.mz, L.mz, R.mz);
+                side(ll.E, left.E, right.E, rr.E, L.E, R.E);
+            }
+            return xg5(face_flux5<SCHEME>(xq5(L), xq5(R), rg, gm1));
+        };
+        double fxl, fxr_;
+        x_factors(i, fxl, fxr_);
         const bool seam_rec_y = MUSCL && ph.periodic_y && true_seam;
         const bool edge_rec_y = MUSCL && ph.periodic_y;
         // z faces: below (k - 1/2) and above (k + 1/2); side A is the lower cell
@@ -283,49 +311,55 @@ __global__ void __launch_bounds__(32 * WPB3, MINB3) stage3_kernel(StageArgs a, i
             V5 unused;
             slope_faces5(limiter, ldrow(jb - 2), uc, un, pc, unused);
         }
+        // Strips of 32 columns: the face on the right of the last one, one row per lane
+        // (in strips of 31 lane 31 forms it in every row).
+        const bool edge = width == 32;
+        if (edge && i0 + 32 <= g.nx && lane < je - jb) {
+            double fl, fr;
+            x_factors(i0 + 32, fl, fr);
+            const double* __restrict__ c = uin + cidx3(g, i0 + 32, jb + lane, k);
+            const V5 f = x_flux(c, toV5(load5(c, P, -1)), toV5(load5(c, P, 0)), fl, fr);
+            xedge[warp][0][lane] = f.r;
+            xedge[warp][1][lane] = f.mx;
+            xedge[warp][2][lane] = f.my;
+            xedge[warp][3][lane] = f.mz;
+            xedge[warp][4][lane] = f.E;
+        }
+        __syncwarp();
+        // this lane's x face: columns past the grid's last face repeat it
+        const double* __restrict__ xcol = uin + cidx3(g, min(i, g.nx), 0, k);
         V5 gb;  // flux of the y face below row j, grid frame
         for (int j = jb - 1; j < je; ++j) {
             const bool row = j >= jb;  // warp-uniform: the first pass only forms the face below row jb
 
-            // Flux divergence, accumulated as each face is formed: the y face below
-            // (carried), the x faces left and right, the z faces below and above,
-            // then the y face above.  The reference sums an interior cell's faces in
+            // Flux divergence, accumulated as each pair of faces is formed (multiply-adds,
+            // rounded explicitly): the y face below (carried), the x faces left and
+            // right, the z faces below and above, then the y face above.  The reference sums an interior cell's faces in
             // for_each_face order (z below, y below, x left, +x, +y, +z;
             // crates/cfd_solver/src/lib.rs:333-337); the order here keeps at most
             // one face flux live at a time and differs from it only in rounding.
             double acc[5];
             if (row) {
                 // ---- x faces on the left and right of column i ----
-                V5 ul = shfl_up5(uc, 1), ur = shfl_down5(uc, 1);
-                V5 ull = ul;
-                if (lane == 0) {
-                    ul = toV5(ld(i0 - 1, j, k));
-                    if (MUSCL) ull = toV5(ld(i0 - 2, j, k));
-                }
-                if (MUSCL && lane == 31) ur = toV5(ld(min(i0 + 32, g.nx + NG - 1), j, k));
-                Q5<double> xl = xq5(ul), xr = xq5(uc);
+                const double* __restrict__ xc = xcol + (long long)j * g.pitch;
+                V5 ul;
                 if (MUSCL) {
-                    V5 pp, mm;
-                    slope_faces5(limiter, ul, uc, ur, pp, mm);
-                    V5 lp = shfl_up5(pp, 1);
-                    if (lane == 0) {
-                        V5 unused;
-                        slope_faces5(limiter, ull, ul, uc, lp, unused);
-                    }
-                    xl = xq5(rec_l ? lp : ul);
-                    xr = xq5(rec_r ? mm : uc);
+                    ul = toV5(load5(xc, P, -1));
+                } else {  // first order reads no other neighbour: a shuffle instead of loads
+                    ul = shfl_up5(uc, 1);
+                    if (lane == 0) ul = toV5(load5(xc, P, -1));
                 }
-                const V5 fx = xg5(face_flux5<SCHEME, double>(xl, xr, rg, gm1));
-                const V5 fxr = shfl_down5(fx, 1);
+                const V5 fx = x_flux(xc, ul, uc, fxl, fxr_);
+                V5 fxr = shfl_down5(fx, 1);
+                if (edge && lane == 31)
+                    fxr = V5{xedge[warp][0][j - jb], xedge[warp][1][j - jb], xedge[warp][2][j - jb],
+                             xedge[warp][3][j - jb], xedge[warp][4][j - jb]};
                 const double yb[5] = {gb.r, gb.mx, gb.my, gb.mz, gb.E};
                 const double fl[5] = {fx.r, fx.mx, fx.my, fx.mz, fx.E};
                 const double fr[5] = {fxr.r, fxr.mx, fxr.my, fxr.mz, fxr.E};
 #pragma unroll
-                for (int v = 0; v < 5; ++v) {
-                    double t = __dmul_rn(yb[v], g.inv_y);
-                    t = __dadd_rn(t, __dmul_rn(fl[v], g.inv_x));
-                    acc[v] = __dsub_rn(t, __dmul_rn(fr[v], g.inv_x));
-                }
+                for (int v = 0; v < 5; ++v)
+                    acc[v] = __fma_rn(__dsub_rn(fl[v], fr[v]), g.inv_x, __dmul_rn(yb[v], g.inv_y));
 
                 // ---- z faces.  One non-unrolled loop marches the column up through
                 // the cells whose z slope this warp limits: its own, and for warp 0
@@ -374,7 +408,7 @@ __global__ void __launch_bounds__(32 * WPB3, MINB3) stage3_kernel(StageArgs a, i
 #pragma unroll 1
                 for (int s = warp == 0 ? 0 : 1; s < 2; ++s) {
                     const V5 L = get(0, warp + s), Rv = get(1, warp + s);
-                    const V5 f = zg5(face_flux5<SCHEME, double>(zq5(L), zq5(Rv), rg, gm1));
+                    const V5 f = zg5(face_flux5<SCHEME>(zq5(L), zq5(Rv), rg, gm1));
                     if (s) fza = f;
                     else fzb = f;
                 }
@@ -390,16 +424,14 @@ __global__ void __launch_bounds__(32 * WPB3, MINB3) stage3_kernel(StageArgs a, i
                 const double zb[5] = {fzb.r, fzb.mx, fzb.my, fzb.mz, fzb.E};
                 const double za[5] = {fza.r, fza.mx, fza.my, fza.mz, fza.E};
 #pragma unroll
-                for (int v = 0; v < 5; ++v) {  // in through the face below, out through the one above
-                    acc[v] = __dadd_rn(acc[v], __dmul_rn(zb[v], g.inv_z));
-                    acc[v] = __dsub_rn(acc[v], __dmul_rn(za[v], g.inv_z));
-                }
+                for (int v = 0; v < 5; ++v)  // in through the face below, out through the one above
+                    acc[v] = __fma_rn(__dsub_rn(zb[v], za[v]), g.inv_z, acc[v]);
             }
 
             // ---- y face above row j ----
             const V5 un2 = ldrow(j + 2);
             V5 pn = un;
-            Q5<double> yb_, yt_;
+            Q5 yb_, yt_;
             if (MUSCL) {
                 V5 mn;
                 slope_faces5(limiter, uc, un, un2, pn, mn);
@@ -412,7 +444,7 @@ __global__ void __launch_bounds__(32 * WPB3, MINB3) stage3_kernel(StageArgs a, i
                 yb_ = yq5(uc);
                 yt_ = yq5(un);
             }
-            const V5 gt = yg5(face_flux5<SCHEME, double>(yb_, yt_, rg, gm1));
+            const V5 gt = yg5(face_flux5<SCHEME>(yb_, yt_, rg, gm1));
 
             if (row && owner && act) {
                 const long long o = cidx3(g, i, j, k);
@@ -420,7 +452,7 @@ __global__ void __launch_bounds__(32 * WPB3, MINB3) stage3_kernel(StageArgs a, i
                 const double yt[5] = {gt.r, gt.mx, gt.my, gt.mz, gt.E};
                 double rhs[5];
 #pragma unroll
-                for (int v = 0; v < 5; ++v) rhs[v] = __dsub_rn(acc[v], __dmul_rn(yt[v], g.inv_y));
+                for (int v = 0; v < 5; ++v) rhs[v] = __fma_rn(-yt[v], g.inv_y, acc[v]);
                 const bool ibm = a.mask != nullptr;
                 const bool solid = ibm && a.mask[o];
                 if (VISC && !solid) {
@@ -501,11 +533,10 @@ __global__ void __launch_bounds__(32 * WPB3, MINB3) stage3_kernel(StageArgs a, i
                     const double w1 = a.stage == 1 ? 0.25 : (2.0 / 3.0);
 #pragma unroll
                     for (int v = 0; v < 5; ++v)
-                        nwv[v] = __dadd_rn(__dmul_rn(w0, a.u0[v * P + o]),
-                                           __dmul_rn(w1, __dadd_rn(ucv[v], __dmul_rn(rhs[v], dt))));
+                        nwv[v] = __fma_rn(w1, __fma_rn(rhs[v], dt, ucv[v]), __dmul_rn(w0, a.u0[v * P + o]));
                 } else {
 #pragma unroll
-                    for (int v = 0; v < 5; ++v) nwv[v] = __dadd_rn(ucv[v], __dmul_rn(rhs[v], dt));
+                    for (int v = 0; v < 5; ++v) nwv[v] = __fma_rn(rhs[v], dt, ucv[v]);
                 }
                 U5 nwu{nwv[0], nwv[1], nwv[2], nwv[3], nwv[4]};
                 if (a.completes_step && ph.sponge) {
@@ -843,25 +874,17 @@ __global__ void __launch_bounds__(IBM_THREADS) ibm3_kernel(Geometry g, Physics p
 }
 
 // ---- launches ---------------------------------------------------------------
-// Rows per warp of the 3-D stage: the fewest that fill the resident slots in one
-// wave, clamped to [2, 12].  A sweep at 256^3 over 4-16 rows and 3-5 resident
-// blocks per SM measured 12 rows and 4 blocks fastest (6.53 ms per inviscid step
-// against 6.65 at 8 rows; 3 and 5 blocks 15 % and 10 % slower).
-static int rows_per_warp3(int nx, int ny, int nz) {
-    const long long strips = (nx + STRIP - 1) / STRIP;
-    const long long slots = 148LL * MINB3 * WPB3;
-    long long rows = (strips * ny * nz + slots - 1) / slots;
-    if (rows < 2) rows = 2;
-    if (rows > 12) rows = 12;
-    return (int)rows;
-}
+// Columns a warp owns (stage3_kernel): 32 where that saves a strip of an inviscid
+// mesh, else 31.
+static int strip_width3(int nx, bool visc) { return !visc && (nx + 31) / 32 < (nx + 30) / 31 ? 32 : 31; }
 
 template <int SCHEME, int RECON, bool VISC, int LIM, bool PXYZ>
 static void launch_stage3_k(const StageArgs& a, bool pdl, cudaStream_t s) {
-    const int rows = rows_per_warp3(a.g.nx, a.g.ny, a.g.nz);
-    const long long blocks = (long long)((a.g.nx + STRIP - 1) / STRIP) * ((a.g.nz + WPB3 - 1) / WPB3);
-    dim3 grid((unsigned)blocks, (a.g.ny + rows - 1) / rows);
-    launch_k(stage3_kernel<SCHEME, RECON, VISC, LIM, PXYZ>, grid, dim3(32 * WPB3), s, pdl, a, rows);
+    const int width = strip_width3(a.g.nx, VISC);
+    const long long across = (long long)((a.g.nx + width - 1) / width) * ((a.g.nz + WPB3 - 1) / WPB3);
+    const int rows = pick_rows(across, a.g.ny, 148LL * MINB3, 2, ROWS3, 0.15);
+    dim3 grid((unsigned)across, (a.g.ny + rows - 1) / rows);
+    launch_k(stage3_kernel<SCHEME, RECON, VISC, LIM, PXYZ>, grid, dim3(32 * WPB3), s, pdl, a, rows, width);
 }
 
 // The inviscid forms are built per limiter (MUSCL) and for fully periodic

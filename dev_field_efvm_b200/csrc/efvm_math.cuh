@@ -331,130 +331,116 @@ __device__ __forceinline__ Q4<R> face_flux(const Q4<R>& L, const Q4<R>& Rr, R ga
 }
 
 // ---- 3-D: states (rho, m_n, m_t, m_s, E) in the frame of the face normal,
-// with two tangential momenta.  The same forms as the 2-D functions above,
+// with two tangential momenta.  The same forms as the FP64 functions above,
 // with the second tangential velocity in |v|^2, the Thornber blend and the
 // star state.
-template <class R>
 struct Q5 {
-    R r, mn, mt, ms, E;
+    double r, mn, mt, ms, E;
 };
-template <class R>
 struct Side5 {
-    R inv, un, ut, us, q, p, a;
+    double un, ut, us, q, p, a2, a;
 };
-template <class R>
-__device__ __forceinline__ Side5<R> side5_with(const Q5<R>& u, R inv, R gamma, R gm1) {
-    Side5<R> s;
-    s.inv = inv;
-    s.un = u.mn * s.inv;
-    s.ut = u.mt * s.inv;
-    s.us = u.ms * s.inv;
-    s.q = s.un * s.un + s.ut * s.ut + s.us * s.us;
-    s.p = gm1 * (u.E - R(0.5) * u.r * s.q);
-    const R a2 = gamma * s.p * s.inv;
-    s.a = a2 * rsqrt_(a2);
+__device__ __forceinline__ Side5 side5(const Q5& u, double inv, double gamma, double gm1) {
+    Side5 s;
+    s.un = __dmul_rn(u.mn, inv);
+    s.ut = __dmul_rn(u.mt, inv);
+    s.us = __dmul_rn(u.ms, inv);
+    s.q = __fma_rn(s.un, s.un, __fma_rn(s.ut, s.ut, __dmul_rn(s.us, s.us)));
+    s.p = __dmul_rn(gm1, __fma_rn(__dmul_rn(-0.5, u.r), s.q, u.E));
+    s.a2 = __dmul_rn(__dmul_rn(gamma, s.p), inv);
+    s.a = __dmul_rn(s.a2, rsqrt_(s.a2));
     return s;
 }
-template <class R>
-__device__ __forceinline__ void sides5_of(const Q5<R>& L, const Q5<R>& Rr, R gamma, R gm1, Side5<R>& l,
-                                          Side5<R>& r) {
-    const R w = rcp_(L.r * Rr.r);
-    l = side5_with(L, Rr.r * w, gamma, gm1);
-    r = side5_with(Rr, L.r * w, gamma, gm1);
+__device__ __forceinline__ void sides5(const Q5& L, const Q5& R, double gamma, double gm1, Side5& l, Side5& r) {
+    const double w = rcp_(__dmul_rn(L.r, R.r));
+    l = side5(L, __dmul_rn(R.r, w), gamma, gm1);
+    r = side5(R, __dmul_rn(L.r, w), gamma, gm1);
 }
 // physical_flux_inline along the face normal, crates/cfd_riemann/src/lib.rs:21-43
-template <class R>
-__device__ __forceinline__ Q5<R> physical_flux5(R rho, R un, R ut, R us, R E, R p) {
-    const R m = rho * un;
-    Q5<R> f;
-    f.r = m;
-    f.mn = m * un + p;
-    f.mt = (rho * ut) * un;
-    f.ms = (rho * us) * un;
-    f.E = (E + p) * un;
+__device__ __forceinline__ Q5 physical_flux5(double rho, double un, double ut, double us, double E, double p) {
+    Q5 f;
+    f.r = __dmul_rn(rho, un);
+    f.mn = __fma_rn(f.r, un, p);
+    f.mt = __dmul_rn(f.r, ut);
+    f.ms = __dmul_rn(f.r, us);
+    f.E = __dmul_rn(__dadd_rn(E, p), un);
     return f;
 }
 // Rusanov::flux_inline, crates/cfd_riemann/src/lib.rs:222-240
-template <class R>
-__device__ __forceinline__ Q5<R> rusanov_flux5(const Q5<R>& L, const Q5<R>& Rr, R gamma, R gm1) {
-    Side5<R> l, r;
-    sides5_of(L, Rr, gamma, gm1, l, r);
-    const Q5<R> fl = physical_flux5(L.r, l.un, l.ut, l.us, L.E, l.p);
-    const Q5<R> fr = physical_flux5(Rr.r, r.un, r.ut, r.us, Rr.E, r.p);
-    const R hl = R(0.5) * fmax_(fabs_(l.un) + l.a, fabs_(r.un) + r.a);
-    Q5<R> f;
-    f.r = R(0.5) * (fl.r + fr.r) - hl * (Rr.r - L.r);
-    f.mn = R(0.5) * (fl.mn + fr.mn) - hl * (Rr.mn - L.mn);
-    f.mt = R(0.5) * (fl.mt + fr.mt) - hl * (Rr.mt - L.mt);
-    f.ms = R(0.5) * (fl.ms + fr.ms) - hl * (Rr.ms - L.ms);
-    f.E = R(0.5) * (fl.E + fr.E) - hl * (Rr.E - L.E);
-    return f;
+__device__ __forceinline__ Q5 rusanov_flux5(const Q5& L, const Q5& R, double gamma, double gm1) {
+    Side5 l, r;
+    sides5(L, R, gamma, gm1, l, r);
+    const Q5 fl = physical_flux5(L.r, l.un, l.ut, l.us, L.E, l.p);
+    const Q5 fr = physical_flux5(R.r, r.un, r.ut, r.us, R.E, r.p);
+    const double hl = __dmul_rn(-0.5, fmax(__dadd_rn(fabs(l.un), l.a), __dadd_rn(fabs(r.un), r.a)));
+    auto mix = [&](double a, double b, double ul, double ur) {
+        return __fma_rn(hl, __dsub_rn(ur, ul), __dmul_rn(0.5, __dadd_rn(a, b)));
+    };
+    return Q5{mix(fl.r, fr.r, L.r, R.r), mix(fl.mn, fr.mn, L.mn, R.mn), mix(fl.mt, fr.mt, L.mt, R.mt),
+              mix(fl.ms, fr.ms, L.ms, R.ms), mix(fl.E, fr.E, L.E, R.E)};
 }
 // Hllc::flux_with_thornber + thornber_reconstruct + star_state,
 // crates/cfd_riemann/src/lib.rs:395-506,619-644, in the equivalent form of
-// hllc_flux above (Thornber over all three velocity components).
-template <class R, bool THORNBER>
-__device__ __forceinline__ Q5<R> hllc_flux5(const Q5<R>& L, const Q5<R>& Rr, R gamma, R gm1) {
-    Side5<R> l, r;
-    sides5_of(L, Rr, gamma, gm1, l, r);
-    R lcn = l.un, lct = l.ut, lcs = l.us, rcn = r.un, rct = r.ut, rcs = r.us, ELc = L.E, ERc = Rr.E;
+// hllc_flux_d above (Thornber over all three velocity components).
+template <bool THORNBER>
+__device__ __forceinline__ Q5 hllc_flux5(const Q5& L, const Q5& R, double gamma, double gm1) {
+    Side5 l, r;
+    sides5(L, R, gamma, gm1, l, r);
+    double lcn = l.un, lct = l.ut, lcs = l.us, rcn = r.un, rct = r.ut, rcs = r.us, ELc = L.E, ERc = R.E;
     if (THORNBER) {
-        const R vmax2 = fmax_(l.q, r.q);
-        const R amax = fmax_(l.a, r.a);
-        const R amax2 = amax * amax;
-        const R prod = vmax2 * amax2;  // below the normal range: z = 0, as in hllc_flux
-        const R z = (vmax2 >= amax2) ? R(1) : (prod >= normal_min<R>() ? vmax2 * rsqrt_(prod) : R(0));
-        const R avgn = R(0.5) * (l.un + r.un), avgt = R(0.5) * (l.ut + r.ut), avgs = R(0.5) * (l.us + r.us);
-        const R hz = R(0.5) * z;
-        const R dvn = hz * (l.un - r.un), dvt = hz * (l.ut - r.ut), dvs = hz * (l.us - r.us);
-        lcn = avgn + dvn;
-        lct = avgt + dvt;
-        lcs = avgs + dvs;
-        rcn = avgn - dvn;
-        rct = avgt - dvt;
-        rcs = avgs - dvs;
-        ELc = L.E + R(0.5) * L.r * ((lcn * lcn + lct * lct + lcs * lcs) - l.q);
-        ERc = Rr.E + R(0.5) * Rr.r * ((rcn * rcn + rct * rct + rcs * rcs) - r.q);
+        const double vmax2 = l.q > r.q ? l.q : r.q;
+        const double amax2 = l.a2 > r.a2 ? l.a2 : r.a2;
+        const double prod = __dmul_rn(vmax2, amax2);  // below the normal range: z = 0, as in hllc_flux_d
+        double hz = __dmul_rn(__dmul_rn(0.5, vmax2), rsqrt_(prod));
+        hz = prod >= normal_min<double>() ? hz : 0.0;
+        hz = vmax2 >= amax2 && amax2 > 0.0 ? 0.5 : hz;
+        auto blend = [&](double a, double b, double& x, double& y) {
+            const double avg = __dmul_rn(0.5, __dadd_rn(a, b)), d = __dsub_rn(a, b);
+            x = __fma_rn(hz, d, avg);
+            y = __fma_rn(-hz, d, avg);
+        };
+        blend(l.un, r.un, lcn, rcn);
+        blend(l.ut, r.ut, lct, rct);
+        blend(l.us, r.us, lcs, rcs);
+        ELc = __fma_rn(__dmul_rn(0.5, L.r), __fma_rn(lcn, lcn, __fma_rn(lct, lct, __fma_rn(lcs, lcs, -l.q))), L.E);
+        ERc = __fma_rn(__dmul_rn(0.5, R.r), __fma_rn(rcn, rcn, __fma_rn(rct, rct, __fma_rn(rcs, rcs, -r.q))), R.E);
     }
-    const R s_l = fmin_(lcn - l.a, rcn - r.a);
-    const R s_r = fmax_(lcn + l.a, rcn + r.a);
-    const R fac_l = L.r * (s_l - lcn);
-    const R fac_r = Rr.r * (s_r - rcn);
-    const R num = (r.p - l.p) + fac_l * lcn - fac_r * rcn;
-    const R den = fac_l - fac_r;
-    const bool star_nonneg = den > R(0) ? num >= R(0) : (den < R(0) ? num <= R(0) : false);
-    const bool useL = (s_l >= R(0)) || star_nonneg;
-    const R rK = useL ? L.r : Rr.r;
-    const R uK = useL ? lcn : rcn;
-    const R tK = useL ? lct : rct;
-    const R sK2 = useL ? lcs : rcs;
-    const R EK = useL ? ELc : ERc;
-    const R pK = useL ? l.p : r.p;
-    const R iK = useL ? l.inv : r.inv;
-    Q5<R> f = physical_flux5(rK, uK, tK, sK2, EK, pK);
-    if (s_l < R(0) && (star_nonneg || s_r >= R(0))) {
-        const R sK = useL ? s_l : s_r;
-        const R facK = useL ? fac_l : fac_r;
-        const R X = facK * (sK * den - num);
-        const R w = rcp_(den * X);
-        const R s_star = num * (X * w);
-        const R dK = sK - s_star;
-        const R inv = den * den * w;
-        const R rho_star = facK * facK * inv;
-        const R e_star = EK * iK + (s_star - uK) * (s_star + pK * dK * inv);
-        f.r = f.r + sK * (rho_star - rK);
-        f.mn = f.mn + sK * (rho_star * s_star - rK * uK);
-        f.mt = f.mt + sK * (rho_star * tK - rK * tK);
-        f.ms = f.ms + sK * (rho_star * sK2 - rK * sK2);
-        f.E = f.E + sK * (rho_star * e_star - EK);
+    const double s_l = fmin(__dsub_rn(lcn, l.a), __dsub_rn(rcn, r.a));
+    const double s_r = fmax(__dadd_rn(lcn, l.a), __dadd_rn(rcn, r.a));
+    const double fac_l = __dmul_rn(L.r, __dsub_rn(s_l, lcn));
+    const double fac_r = __dmul_rn(R.r, __dsub_rn(s_r, rcn));
+    const double num = __fma_rn(-fac_r, rcn, __fma_rn(fac_l, lcn, __dsub_rn(r.p, l.p)));
+    const double den = __dsub_rn(fac_l, fac_r);
+    const bool star_nonneg = __dmul_rn(num, den) >= 0.0 && den != 0.0;
+    const bool useL = (s_l >= 0.0) || star_nonneg;
+    const double uK = useL ? lcn : rcn;
+    const double tK = useL ? lct : rct;
+    const double wK = useL ? lcs : rcs;
+    const double EK = useL ? ELc : ERc;
+    const double pK = useL ? l.p : r.p;
+    if (s_l < 0.0 && (star_nonneg || s_r >= 0.0)) {
+        const double sK = useL ? s_l : s_r;
+        const double facK = useL ? fac_l : fac_r;
+        const double Y = __fma_rn(sK, den, -num);
+        const double w = rcp_(__dmul_rn(den, Y));
+        const double s_star = __dmul_rn(num, __dmul_rn(Y, w));
+        const double inv = __dmul_rn(den, __dmul_rn(den, w));  // 1 / (s_K - s_*)
+        const double pS = __fma_rn(facK, __dsub_rn(s_star, uK), pK);
+        Q5 f;
+        f.r = __dmul_rn(__dmul_rn(facK, inv), s_star);
+        f.mn = __fma_rn(f.r, s_star, pS);
+        f.mt = __dmul_rn(f.r, tK);
+        f.ms = __dmul_rn(f.r, wK);
+        const double eS = __fma_rn(pS, s_star, __fma_rn(__dsub_rn(sK, uK), EK, -__dmul_rn(pK, uK)));
+        f.E = __dmul_rn(__fma_rn(eS, inv, pS), s_star);
+        return f;
     }
-    return f;
+    return physical_flux5(useL ? L.r : R.r, uK, tK, wK, EK, pK);
 }
-template <int SCHEME, class R>
-__device__ __forceinline__ Q5<R> face_flux5(const Q5<R>& L, const Q5<R>& Rr, R gamma, R gm1) {
-    if (SCHEME == EFVM_FLUX_RUSANOV) return rusanov_flux5(L, Rr, gamma, gm1);
-    if (SCHEME == EFVM_FLUX_HLLC_TEXTBOOK) return hllc_flux5<R, false>(L, Rr, gamma, gm1);
-    return hllc_flux5<R, true>(L, Rr, gamma, gm1);
+template <int SCHEME>
+__device__ __forceinline__ Q5 face_flux5(const Q5& L, const Q5& R, double gamma, double gm1) {
+    if (SCHEME == EFVM_FLUX_RUSANOV) return rusanov_flux5(L, R, gamma, gm1);
+    return hllc_flux5<SCHEME != EFVM_FLUX_HLLC_TEXTBOOK>(L, R, gamma, gm1);
 }
 
 // minmod / monotonized_central, crates/cfd_solver/src/lib.rs:170-192.  (Deciding
