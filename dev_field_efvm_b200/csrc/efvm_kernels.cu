@@ -114,6 +114,11 @@ struct TmaSrc {
         const double* p = row(jj) + (ii - col0);
         return U4{p[0], p[tma::IN_COLS], p[2 * tma::IN_COLS], p[3 * tma::IN_COLS]};
     }
+    // this lane's column + d (-2 .. 1; the slot holds two halo columns on each side)
+    __device__ __forceinline__ U4 beside(int jj, int d) const {
+        const double* p = row(jj) + scol + d;
+        return U4{p[0], p[tma::IN_COLS], p[2 * tma::IN_COLS], p[3 * tma::IN_COLS]};
+    }
     const double* u0;           // U^n in global memory (when the ring holds no U^n rows)
     long long plane;
     __device__ __forceinline__ double u0v(int v, long long o, int i, int j) const {
@@ -195,6 +200,7 @@ __device__ __forceinline__ void stage_strip_src(const A& a, int rows, int strip,
         if constexpr (CG) machine((volatile DevState*)a.st);
         else machine(a.st);
     }
+    constexpr bool BATCH = !std::is_same<A, StageArgs>::value;
     const int i0 = strip * STRIP;
     const int jb = by * rows;
     double lam = 0.0;
@@ -217,13 +223,15 @@ __device__ __forceinline__ void stage_strip_src(const A& a, int rows, int strip,
         // What a lane carries from one row to the next (the flux of the y face
         // below the row, in the face frame, and the row's +y face state) and,
         // within a row, the x part of the flux divergence while the y face is
-        // formed.  The FP32-flux forms keep them in registers.  The FP64 forms
-        // keep them in shared memory, one slot per thread (12 doubles, 12 KB per
+        // formed.  The FP32-flux forms keep them in registers.  The FP64 strip form
+        // keeps them in shared memory, one slot per thread (12 doubles, 12 KB per
         // block): that frees 24 registers through both flux evaluations, halves
-        // the FP64 inviscid form's spills, and took the 4096^2 FP64 strip step
-        // from 2.73 to 2.58 ms (FP32 fluxes, TMA form: 1.73 -> 1.90 ms, so not
-        // there).
-        constexpr bool CARRY_GB = FP64, CARRY_PC = FP64, CARRY_PART = FP64;
+        // its spills, and took its 4096^2 step from 2.73 to 2.58 ms (FP32 fluxes,
+        // TMA form: 1.73 -> 1.90 ms, so not there).  The FP64 TMA-fed form, whose x
+        // faces hold no shuffled states, keeps only the flux there (4 KB): 1.709
+        // against 1.722 ms per 4096^2 step with all three, 1.718 with none.
+        constexpr bool TMA = std::is_same<SRC, TmaSrc>::value;
+        constexpr bool CARRY_GB = FP64, CARRY_PC = FP64 && !TMA, CARRY_PART = FP64 && !TMA;
         constexpr int SLOT_GB = 0, SLOT_PC = SLOT_GB + (CARRY_GB ? 4 : 0), SLOT_PART = SLOT_PC + (CARRY_PC ? 4 : 0);
         constexpr int CARRY_SLOTS = SLOT_PART + (CARRY_PART ? 4 : 0);
         __shared__ double carry_s[CARRY_SLOTS > 0 ? CARRY_SLOTS : 1][32 * WPB];
@@ -242,6 +250,9 @@ __device__ __forceinline__ void stage_strip_src(const A& a, int rows, int strip,
             rec_l = ph.periodic_x;
             rec_r = ph.periodic_x && true_seam;
         }
+        // the same as slope factors (the high words of 0.5 and 0; FP64 TMA-fed form)
+        const bool x_edge = i < NG || i >= g.nx - NG;
+        const int fxl = rec_l ? 0x3fe00000 : 0, fxr_ = rec_r ? 0x3fe00000 : 0;
         const bool y_periodic = ph.periodic_y || ph.seam_ylo || ph.seam_yhi;
         const bool seam_rec = y_periodic && true_seam;  // the side across the periodic seam
         const bool edge_rec = y_periodic;               // the side inside the domain
@@ -251,11 +262,13 @@ __device__ __forceinline__ void stage_strip_src(const A& a, int rows, int strip,
         // read where they are used: hoisted out of the loop they made the batch
         // kernels, whose physics is read from the case table, 6 % slower.)
         auto rec_below = [&](int jj) {
+            if constexpr (PXY) return jj == -1 ? true_seam : true;  // whole periodic grids: no slab edges
             const bool lo_edge_rows = !ph.halo_ylo || ph.seam_ylo, hi_edge_rows = !ph.halo_yhi || ph.seam_yhi;
             const bool lo = jj == -1 && lo_edge_rows, hi = jj + 1 == g.ny && hi_edge_rows;
             return lo ? seam_rec : (hi ? edge_rec : true);
         };
         auto rec_above = [&](int jj) {
+            if constexpr (PXY) return jj + 1 == g.ny ? true_seam : true;
             const bool lo_edge_rows = !ph.halo_ylo || ph.seam_ylo, hi_edge_rows = !ph.halo_yhi || ph.seam_yhi;
             const bool lo = jj == -1 && lo_edge_rows, hi = jj + 1 == g.ny && hi_edge_rows;
             return lo ? edge_rec : (hi ? seam_rec : true);
@@ -283,6 +296,8 @@ __device__ __forceinline__ void stage_strip_src(const A& a, int rows, int strip,
         }
         src.release(jb - 2);
         const double dt = gld<CG>(&a.st->dt);  // set by the step's set-up, constant during the stage
+        const double w0 = a.stage == 1 ? 0.75 : (1.0 / 3.0);  // RK weights of stages 2 and 3
+        const double w1 = a.stage == 1 ? 0.25 : (2.0 / 3.0);
         Q4<R> gb{R(0), R(0), R(0), R(0)};
         // carry slots: gb (r, mn, mt, E), pc (r, mx, my, E), the x part (4 planes)
         auto put_gb = [&](const Q4<R>& q) {
@@ -313,6 +328,10 @@ __device__ __forceinline__ void stage_strip_src(const A& a, int rows, int strip,
                              carry_s[SLOT_PC + 3][tq]};
             else return pc;
         };
+        // The FP32-flux TMA-fed form carries the flux widened, as its epilogue uses
+        // it: each flux is converted once (4096^2: 1.454 -> 1.445 ms per step).
+        constexpr bool CARRY_WIDE = !FP64 && TMA;
+        double gb_wide[CARRY_WIDE ? 4 : 1] = {};
         put_gb(gb);
         if (MUSCL) put_pc(pc);
         for (int j = jb - 1; rows_ok && j < je; ++j) {
@@ -323,7 +342,7 @@ __device__ __forceinline__ void stage_strip_src(const A& a, int rows, int strip,
             // row: with the carry in shared memory that left it no spills at 80
             // registers, and took the 4096^2 vortex from 2.64 (strip form) to
             // 2.26 ms per step.  The other forms hold them in registers.
-            constexpr bool REREAD = FP64 && std::is_same<SRC, TmaSrc>::value;
+            constexpr bool REREAD = FP64 && TMA;
             const V4<R> un2 = REREAD ? V4<R>{} : ldrow(j + 2);
             auto row_c = [&]() { if constexpr (REREAD) return ldrow(j); else return uc; };
             auto row_n = [&]() { if constexpr (REREAD) return ldrow(j + 1); else return un; };
@@ -349,27 +368,57 @@ __device__ __forceinline__ void stage_strip_src(const A& a, int rows, int strip,
                 else return part_r[v];
             };
             auto x_face = [&]() {
-                V4<R> ul = shfl_up_v(row_c(), 1), ur = shfl_down_v(row_c(), 1);
-                V4<R> ull = ul;  // column i-2 (lane 0 only)
-                if (lane == 0) {
-                    ul = toR<R>(ld(i0 - 1, j));
-                    if (MUSCL) ull = toR<R>(ld(i0 - 2, j));
-                }
-                if (MUSCL && lane == 31) ur = toR<R>(ld(min(i0 + 32, g.nx + NG - 1), j));
                 Q4<R> fx;
-                if (MUSCL) {
-                    V4<R> pp, mm;  // this column's +x and -x face states
-                    if constexpr (FP64) slope_faces(limiter, ul, row_c(), ur, R(0.5), R(0.5), pp, mm);
-                    else slope_faces_half(limiter, ul, row_c(), ur, pp, mm);
-                    V4<R> lp = shfl_up_v(pp, 1);  // +x state of column i-1
-                    if (lane == 0) {
-                        V4<R> unused;
-                        if constexpr (FP64) slope_faces(limiter, ull, ul, row_c(), R(0.5), R(0), lp, unused);
-                        else slope_faces_half(limiter, ull, ul, row_c(), lp, unused);
-                    }
-                    fx = face_flux<SCHEME, R>(xq(rec_l ? lp : ul), xq(rec_r ? mm : row_c()), rg, rgm1);
+                if constexpr (MUSCL && TMA) {
+                    // Both slopes of the face from the four cells about it in the
+                    // ring: 12 more shared loads and 4 more slopes than with
+                    // shuffled neighbours, against 24 shuffles, lane 0's extra slope
+                    // and the halo loads of lanes 0 and 31 in every row (4096^2:
+                    // 1.836 -> 1.722 ms per FP64 step; FP32 fluxes the same time at
+                    // 7 registers less, 512^2 55 -> 51 us).
+                    const V4<R> q0 = toR<R>(src.beside(j, -2)), q1 = toR<R>(src.beside(j, -1)), q2 = row_c(),
+                                q3 = toR<R>(src.beside(j, 1));
+                    V4<R> l, r;
+                    auto side = [&](R c0, R c1, R c2, R c3, R& lo, R& hi) {
+                        if constexpr (FP64) {
+                            const double d1 = c1 - c0, d2 = c2 - c1, d3 = c3 - c2;
+                            double sl, f;
+                            limited_slope(limiter, d2, d1, __hiloint2double(fxl, 0), sl, f);
+                            lo = fma(sl, f, c1);
+                            limited_slope(limiter, d3, d2, __hiloint2double(fxr_, 0), sl, f);
+                            hi = fma(-sl, f, c2);
+                        } else {
+                            lo = rec_l ? c1 + half_slope(limiter, c0, c1, c2) : c1;
+                            hi = rec_r ? c2 - half_slope(limiter, c1, c2, c3) : c2;
+                        }
+                    };
+                    side(q0.r, q1.r, q2.r, q3.r, l.r, r.r);
+                    side(q0.mx, q1.mx, q2.mx, q3.mx, l.mx, r.mx);
+                    side(q0.my, q1.my, q2.my, q3.my, l.my, r.my);
+                    side(q0.E, q1.E, q2.E, q3.E, l.E, r.E);
+                    fx = face_flux<SCHEME, R, BATCH>(xq(l), xq(r), rg, rgm1);
                 } else {
-                    fx = face_flux<SCHEME, R>(xq(ul), xq(row_c()), rg, rgm1);
+                    V4<R> ul = shfl_up_v(row_c(), 1), ur = shfl_down_v(row_c(), 1);
+                    V4<R> ull = ul;  // column i-2 (lane 0 only)
+                    if (lane == 0) {
+                        ul = toR<R>(ld(i0 - 1, j));
+                        if (MUSCL) ull = toR<R>(ld(i0 - 2, j));
+                    }
+                    if (MUSCL && lane == 31) ur = toR<R>(ld(min(i0 + 32, g.nx + NG - 1), j));
+                    if (MUSCL) {
+                        V4<R> pp, mm;  // this column's +x and -x face states
+                        if constexpr (FP64) slope_faces(limiter, ul, row_c(), ur, R(0.5), R(0.5), pp, mm);
+                        else slope_faces_half(limiter, ul, row_c(), ur, pp, mm);
+                        V4<R> lp = shfl_up_v(pp, 1);  // +x state of column i-1
+                        if (lane == 0) {
+                            V4<R> unused;
+                            if constexpr (FP64) slope_faces(limiter, ull, ul, row_c(), R(0.5), R(0), lp, unused);
+                            else slope_faces_half(limiter, ull, ul, row_c(), lp, unused);
+                        }
+                        fx = face_flux<SCHEME, R, BATCH>(xq(rec_l ? lp : ul), xq(rec_r ? mm : row_c()), rg, rgm1);
+                    } else {
+                        fx = face_flux<SCHEME, R, BATCH>(xq(ul), xq(row_c()), rg, rgm1);
+                    }
                 }
                 const Q4<R> fxr = shfl_down_q(fx, 1);  // face on the right of column i
                 const double fl[4] = {(double)fx.r, (double)fx.mn, (double)fx.mt, (double)fx.E};
@@ -388,13 +437,13 @@ __device__ __forceinline__ void stage_strip_src(const A& a, int rows, int strip,
                 else slope_faces_half(limiter, row_c(), row_n(), row_n2(), pn, mn);
                 put_pc(pn);
                 if constexpr (Y_FACTORS) {
-                    gt = face_flux<SCHEME, R>(yq(pcr), yq(mn), rg, rgm1);
+                    gt = face_flux<SCHEME, R, BATCH>(yq(pcr), yq(mn), rg, rgm1);
                 } else {
                     const bool rb = rec_below(j), rt = rec_above(j);
-                    gt = face_flux<SCHEME, R>(yq(rb ? pcr : row_c()), yq(rt ? mn : row_n()), rg, rgm1);
+                    gt = face_flux<SCHEME, R, BATCH>(yq(rb ? pcr : row_c()), yq(rt ? mn : row_n()), rg, rgm1);
                 }
             } else {
-                gt = face_flux<SCHEME, R>(yq(row_c()), yq(row_n()), rg, rgm1);
+                gt = face_flux<SCHEME, R, BATCH>(yq(row_c()), yq(row_n()), rg, rgm1);
             }
             if (!XFIRST && row) x_face();
 
@@ -403,8 +452,17 @@ __device__ __forceinline__ void stage_strip_src(const A& a, int rows, int strip,
                 // the cell's state in FP64 (the FP32 path reads it again)
                 const U4 ucd = FP64 ? toU4(row_c()) : ld(i, j);
                 const double gtv[4] = {(double)gt.r, (double)gt.mt, (double)gt.mn, (double)gt.E};
-                const Q4<R> gbq = get_gb();
-                const double gbd[4] = {(double)gbq.r, (double)gbq.mt, (double)gbq.mn, (double)gbq.E};
+                double gbd[4];  // the flux below
+                if constexpr (CARRY_WIDE) {
+#pragma unroll
+                    for (int v = 0; v < 4; ++v) gbd[v] = gb_wide[v];
+                } else {
+                    const Q4<R> q = get_gb();
+                    gbd[0] = (double)q.r;
+                    gbd[1] = (double)q.mt;
+                    gbd[2] = (double)q.mn;
+                    gbd[3] = (double)q.E;
+                }
                 double rhs[4];
 #pragma unroll
                 for (int v = 0; v < 4; ++v) rhs[v] = fma(gbd[v] - gtv[v], g.inv_y, get_part(v));
@@ -510,8 +568,6 @@ __device__ __forceinline__ void stage_strip_src(const A& a, int rows, int strip,
                 const double ucv[4] = {ucd.r, ucd.mx, ucd.my, ucd.E};
                 double un_[4];
                 if (a.stage == 1 || a.stage == 2) {
-                    const double w0 = a.stage == 1 ? 0.75 : (1.0 / 3.0);
-                    const double w1 = a.stage == 1 ? 0.25 : (2.0 / 3.0);
 #pragma unroll
                     for (int v = 0; v < 4; ++v) un_[v] = fma(w1, fma(rhs[v], dt, ucv[v]), w0 * src.u0v(v, o, i, j));
                 } else {
@@ -529,7 +585,14 @@ __device__ __forceinline__ void stage_strip_src(const A& a, int rows, int strip,
                 if (a.completes_step && a.want_cfl) lam = fmax(lam, wave_speed(g, ph, nw));
             }
             src.release(j);
-            put_gb(gt);
+            if constexpr (CARRY_WIDE) {
+                gb_wide[0] = (double)gt.r;
+                gb_wide[1] = (double)gt.mt;
+                gb_wide[2] = (double)gt.mn;
+                gb_wide[3] = (double)gt.E;
+            } else {
+                put_gb(gt);
+            }
             uc = un;
             un = un2;
         }
@@ -1369,9 +1432,9 @@ static void launch_stage_r(const StageArgs& a, bool pdl, cudaStream_t s) {
 // ---- the TMA-fed stage kernel ----------------------------------------------
 // Resident blocks per SM.  The FP32-flux form's shared memory is the ring
 // (32.3 KB per block), so six fit in the SM's 228 KB, and it is built for six
-// (80 registers).  The FP64 form adds its 12 KB row carry, so five fit, and it
-// is built for five (up to 102 registers; it uses 92, 1 % faster at 4096^2
-// than the same form held to 80).
+// (80 registers).  The FP64 form adds its 4 KB carry; six would fit, but it is
+// built for five (95 registers: 1.709 ms per 4096^2 step against 1.742 held to
+// 80, where it spills).
 constexpr int TMA_MINB = 6;
 constexpr int tma_resident(bool fp32) { return fp32 ? TMA_MINB : 5; }
 
@@ -1381,7 +1444,7 @@ bool stage_tma_eligible(const Geometry& g, const Physics& ph, bool ibm, bool cor
 
 template <int SCHEME, int RECON, class R, int LIM, bool PXY>
 static void launch_stage_tma_k(const StageArgs& a, bool pdl, cudaStream_t s) {
-    constexpr bool XFIRST = StageForm<R, false>::XFIRST;
+    constexpr bool XFIRST = false;  // FP64: 1.682 against 1.709 ms per 4096^2 step with the x face first
     auto kernel = stage_tma_kernel<SCHEME, RECON, R, tma_resident(sizeof(R) == sizeof(float)), XFIRST, LIM, PXY>;
     // the largest shared-memory carve-out, once per device
     static unsigned long long carveout_set = 0;
