@@ -986,17 +986,21 @@ __device__ __forceinline__ bool sample_bilinear(const Geometry& g, const Physics
     return true;
 }
 
-// Mirror (apply_ibm_ghost_bc, crates/cfd_ibm/src/lib.rs:258-289) of every solid
+// Mirror (apply_ibm_ghost_bc, crates/cfd_ibm/src/lib.rs:258-289) of one solid
 // ghost cell, recording its pre-mirror value for the emulated z-ghost of the
-// staircase wall force.  One thread per ghost cell.
+// staircase wall force.  The step's state (`st`) is read beside the cell's loads
+// and tested before anything is written.
 __device__ __forceinline__ void mirror_ghost(const Geometry& g, const Physics& ph, const Ibm& ib, double* q,
-                                             int stage, int k, int par) {
-    const IbmGhostDev gh = ib.ghosts[k];
+                                             const DevState* st, int stage, int k, const IbmGhostDev& gh, int setup) {
+    const int active = st->active;
+    const int par = (int)(st->step & 1ull);
+    const bool stops = setup && step_stops(st);
     const long long o = cidx(g, gh.i, gh.j);
     const U4 pre = load4(q, g.plane, o);
     double img[5];
     const bool ok = gh.valid && (gh.fluid & GHOST_MIRROR_BIT) &&
                     sample_bilinear(g, ph, q, gh.fluid, gh.lo_i, gh.lo_j, gh.tx, gh.ty, img);
+    if (!active || stops) return;
     double* zf = ib.zfill + ((long long)stage % 3) * ib.n_ghost * 4 + 4LL * k;
     zf[0] = pre.r; zf[1] = pre.mx; zf[2] = pre.my; zf[3] = pre.E;
     if (stage == 0 || stage == 3) {
@@ -1158,23 +1162,27 @@ __device__ __forceinline__ void forces_block(const Geometry& g, const Physics& p
 __global__ void __launch_bounds__(IBM_THREADS) ibm_kernel(Geometry g, Physics ph, Ibm ib, double* q, DevState* st,
                                                           int force_stage, int n_force_blocks, int mirror_stage,
                                                           int setup, int deferred) {
-    pdl_wait_then_release();
     const int b = blockIdx.x;
+    const int k = (b - n_force_blocks) * blockDim.x + threadIdx.x;
+    const bool mirrors = b >= n_force_blocks && mirror_stage >= 0 && k < ib.n_ghost;
+    // the ghost list changes only with the geometry: read ahead of the wait
+    IbmGhostDev gh{};
+    if (mirrors) gh = ib.ghosts[k];
+    pdl_wait_then_release();
     if (b < n_force_blocks) {  // uniform per block
         // Deferred forces belong to a step that ran; they go ahead whatever this
-        // launch's set-up decides, and only while they are pending.  Every block
+        // step's set-up decides, and only while they are pending.  Every block
         // reads the flag before it counts itself in, and only the last one clears it.
         if (deferred ? !st->forces_pending : !st->active) return;
         forces_block(g, ph, ib, q, st, force_stage, b, n_force_blocks, deferred);
         return;
     }
-    if (!st->active) return;
-    if (setup) {
-        if (b == n_force_blocks && threadIdx.x == 0) step_setup(ph, st);
-        if (step_stops(st)) return;
+    if (setup && b == n_force_blocks && threadIdx.x == 0) {
+        // every mirror thread of the launch applies the stop rule itself, whether it
+        // reads the state before this or after (a set-up that stops clears `active`)
+        if (st->active) step_setup(ph, st);
     }
-    const int k = (b - n_force_blocks) * blockDim.x + threadIdx.x;
-    if (mirror_stage >= 0 && k < ib.n_ghost) mirror_ghost(g, ph, ib, q, mirror_stage, k, (int)(st->step & 1ull));
+    if (mirrors) mirror_ghost(g, ph, ib, q, st, mirror_stage, k, gh, setup);
 }
 
 // ---------------------------------------------------------------------------

@@ -731,8 +731,7 @@ __device__ __forceinline__ bool sample_trilinear3(const Geometry& g, const Physi
 // image point's density, pressure and temperature and the velocity mirrored
 // about the wall velocity, 2 u_w - u_image; a ghost whose sample fails keeps its
 // value.
-__device__ __forceinline__ void mirror_ghost3(const Geometry& g, const Physics& ph, const Ibm& ib, double* q, int t) {
-    const IbmGhost3Dev gh = ib.ghosts3[t];
+__device__ __forceinline__ void mirror_ghost3(const Geometry& g, const Physics& ph, double* q, const IbmGhost3Dev& gh) {
     if (!gh.valid) return;
     double im[6];
     if (!sample_trilinear3(g, ph, q, gh.fluid, gh.lo, gh.t, im)) return;
@@ -814,12 +813,15 @@ __device__ __forceinline__ void wall_load3(const Geometry& g, const Physics& ph,
 // stage, run only while they are pending, and then cleared by the last block.
 __global__ void __launch_bounds__(IBM_THREADS) ibm3_kernel(Geometry g, Physics ph, Ibm ib, double* q, DevState* st,
                                                            int nfm, int nf, int setup, int deferred) {
-    pdl_wait_then_release();
     const int b = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int k = (b - nf) * IBM_THREADS + tid;
+    // the ghost list changes only with the geometry: read ahead of the wait
+    IbmGhost3Dev gh{};
+    if (b >= nf && k < ib.n_ghost) gh = ib.ghosts3[k];
+    pdl_wait_then_release();
     if (b >= nf) {  // uniform per block
         if (setup && b == nf && tid == 0 && st->active) step_setup(ph, st);
-        const int t = (b - nf) * IBM_THREADS + tid;
-        if (t < ib.n_ghost) mirror_ghost3(g, ph, ib, q, t);
+        if (k < ib.n_ghost) mirror_ghost3(g, ph, q, gh);
         return;
     }
     // Every block reads the flag before it counts itself in; only the last one clears it.
