@@ -237,14 +237,64 @@ __device__ __forceinline__ void sponge_2d(const Geometry& g, const Physics& ph, 
 // Flags a non-physical state (rho <= 0, p <= 0, NaN).  p > 0 with rho > 0 is
 // 2 E rho > m^2 (no division); a NaN in any component fails one of the two
 // tests, so the NaN bit is only looked at once a test has failed.
-__device__ __forceinline__ void flag_nonphysical(DevState* st, const U4& nw) {
+__device__ __forceinline__ void flag_nonphysical(int* flags, const U4& nw) {
     int bad = 0;
     if (!(nw.r > 0.0)) bad |= 1;
     if (!(2.0 * nw.E * nw.r > nw.mx * nw.mx + nw.my * nw.my)) bad |= 2;
     if (bad) {
         if (nw.r != nw.r || nw.mx != nw.mx || nw.my != nw.my || nw.E != nw.E) bad |= 4;
-        atomicOr(&st->nonphysical, bad);
+        atomicOr(flags, bad);
     }
+}
+
+// Per-step Setup: dt from the wave-speed max (cfl_system's final lines,
+// crates/cfd_solver/src/lib.rs:671-676) or fixed_dt, and the stop test of the
+// case drivers' `if t >= T_FINAL break`.
+// The stop rule of step_setup: a non-physical state or t >= t_stop ends the run.
+template <class S>
+__device__ __forceinline__ bool step_stops(S* st) {
+    return st->nonphysical || (st->stop_at_t && st->time >= st->t_stop);
+}
+
+__device__ __forceinline__ unsigned long long global_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+// The step's dt: cfl / max wave speed (cfl_system, crates/cfd_solver/src/lib.rs:647-669).
+template <class S>
+__device__ __forceinline__ double step_dt(const Physics& ph, const S* st) {
+    if (ph.fixed_dt > 0.0) return ph.fixed_dt;
+    const unsigned long long bits = st->ext_lam ? st->lam_ext : st->lam[st->lam_idx];
+    const double lam = __longlong_as_double((long long)bits);
+    return lam > 0.0 ? ph.cfl / lam : INFINITY;
+}
+// The switch of the wave-speed buffer that the step's last stage accumulates into.
+template <class S>
+__device__ __forceinline__ void switch_lam(S* st) {
+    if (st->ext_lam) {  // the slot starts this step's accumulation from zero
+        st->lam_ext = 0ull;
+        return;
+    }
+    const int nxt = st->lam_idx ^ 1;
+    st->lam[nxt] = 0ull;
+    st->lam_idx = nxt;
+}
+
+// Per-step set-up (one thread): stop check, dt and the wave-speed buffer.
+// S = DevState, or volatile DevState where other blocks of the same launch
+// write the state (the persistent batch kernel).
+template <class S>
+__device__ __forceinline__ void step_setup(const Physics& ph, S* st) {
+    if (step_stops(st)) {
+        st->active = 0;
+        st->done_ns = global_ns();
+        return;
+    }
+    st->dt = step_dt(ph, st);
+    st->step_par = (int)(st->step & 1ull);
+    switch_lam(st);
 }
 
 __device__ __forceinline__ void block_max_atomic(double v, unsigned long long* target) {

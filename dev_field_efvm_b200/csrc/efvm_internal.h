@@ -46,7 +46,8 @@ struct DevState {
     unsigned long long done_ns;  // device global timer when the set-up stopped the run
     int step_par;            // parity of the step in progress (step & 1 at its set-up): the z-ghost
                              // buffer that the forces of its first two stages read
-    int pad_par_;
+    int flags0;              // nonphysical bits of a first stage that does the step's set-up itself
+                             // (its blocks still test `nonphysical`); stage 2 merges them
 };
 
 // Boundary side description resolved for the device.
@@ -208,6 +209,7 @@ struct StageArgs {
     const void* tmap_u0;
     int rows;                         // rows per warp; 0 = the built-in choice
     int tile;                         // 1: the face-parallel kernel (efvm_tile.cu)
+    int fold_setup;                   // face-parallel kernel: stages 1 and 2 do the step's set-up
     int blocks;                       // resident blocks per SM of the strip form; 0 = the built-in choice
     unsigned long long wait_ns;       // limit of one wait of the TMA-fed kernel for a row (ns)
     int stall;                        // failure injection: the first block's ring stops being refilled

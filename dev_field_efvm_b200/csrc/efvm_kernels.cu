@@ -581,7 +581,7 @@ __device__ __forceinline__ void stage_strip_src(const A& a, int rows, int strip,
                 write_ghosts<PXY>(g, ph, a.uout, i, j, nw);
                 peer_rows(a, g, i, j, nw);
 
-                flag_nonphysical(a.st, nw);
+                flag_nonphysical(&a.st->nonphysical, nw);
                 if (a.completes_step && a.want_cfl) lam = fmax(lam, wave_speed(g, ph, nw));
             }
             src.release(j);
@@ -730,52 +730,6 @@ __global__ void cfl_kernel(Geometry g, Physics ph, const double* __restrict__ q,
 
 __global__ void reset_lam_kernel(DevState* st) {
     *lam_slot(st) = 0ull;
-}
-
-// Per-step Setup: dt from the wave-speed max (cfl_system's final lines,
-// crates/cfd_solver/src/lib.rs:671-676) or fixed_dt, and the stop test of the
-// case drivers' `if t >= T_FINAL break`.
-// The stop rule of step_setup: a non-physical state or t >= t_stop ends the run.
-template <class S>
-__device__ __forceinline__ bool step_stops(S* st) {
-    return st->nonphysical || (st->stop_at_t && st->time >= st->t_stop);
-}
-
-// Per-step set-up (one thread): stop check, dt = cfl / max wave speed (cfl_system,
-// crates/cfd_solver/src/lib.rs:647-669) and the switch of the wave-speed buffer
-// that the step's last stage accumulates into.
-__device__ __forceinline__ unsigned long long global_ns() {
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-// S = DevState, or volatile DevState where other blocks of the same launch
-// write the state (the persistent batch kernel).
-template <class S>
-__device__ __forceinline__ void step_setup(const Physics& ph, S* st) {
-    if (step_stops(st)) {
-        st->active = 0;
-        st->done_ns = global_ns();
-        return;
-    }
-    double dt;
-    if (ph.fixed_dt > 0.0) {
-        dt = ph.fixed_dt;
-    } else {
-        const unsigned long long bits = st->ext_lam ? st->lam_ext : st->lam[st->lam_idx];
-        const double lam = __longlong_as_double((long long)bits);
-        dt = lam > 0.0 ? ph.cfl / lam : INFINITY;
-    }
-    st->dt = dt;
-    st->step_par = (int)(st->step & 1ull);
-    if (st->ext_lam) {  // the slot starts this step's accumulation from zero
-        st->lam_ext = 0ull;
-        return;
-    }
-    const int nxt = st->lam_idx ^ 1;
-    st->lam[nxt] = 0ull;
-    st->lam_idx = nxt;
 }
 
 __global__ void step_setup_kernel(Physics ph, DevState* st) {

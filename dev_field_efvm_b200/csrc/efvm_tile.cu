@@ -49,16 +49,42 @@ __global__ void __launch_bounds__(32 * (2 * R + 1), MINB) tile_stage_kernel(cons
     __shared__ double flux[4][W][32];
     // viscous: u, v, T of the tile's cells and the ring around them, row jb - 1 + r, column i0 - 1 + c
     __shared__ double prim[VISC ? 3 : 1][VISC ? R + 2 : 1][VISC ? 34 : 1];
+    const Geometry& g = a.g;
+    const Physics& ph = a.ph;
     pdl_wait_then_release();
     // read ahead of the state's loads, tested after them: a whole stage of a small
     // grid is a few memory latencies and one chain of arithmetic
-    const int active = a.st->active;
-    const double dt = a.st->dt;
-    const Geometry& g = a.g;
-    const Physics& ph = a.ph;
+    // (the viscous forms have no registers to spare and keep the set-up launch)
+    const bool fold = !VISC && a.fold_setup;
+    const bool setup = fold && a.stage == 0;
+    const int active = a.st->active && !(setup && step_stops(a.st));
+    const double dt = setup ? step_dt(ph, a.st) : a.st->dt;
     const long long P = g.plane;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int i0 = blockIdx.x * STRIP, jb = blockIdx.y * R;
+    if (fold && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
+        // The step's set-up (step_setup) without a launch of its own.  In stage 1 every
+        // block forms dt and the stop decision from fields that this launch does not
+        // change -- its own non-physical bits go to flags0 -- and this thread records
+        // them; stage 2 merges the bits and switches the wave-speed buffer, which no
+        // block of it reads.
+        DevState* st = a.st;
+        if (setup) {
+            if (active) {
+                st->dt = dt;
+                st->step_par = (int)(st->step & 1ull);
+            } else if (st->active) {
+                st->active = 0;
+                st->done_ns = global_ns();
+            }
+        } else if (a.stage == 1 && active) {
+            if (st->flags0) {
+                atomicOr(&st->nonphysical, st->flags0);
+                st->flags0 = 0;
+            }
+            switch_lam(st);
+        }
+    }
     if (active && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
         // RK state machine and clock of update_system, crates/cfd_solver/src/lib.rs:607-621
         DevState* st = a.st;
@@ -250,7 +276,7 @@ __global__ void __launch_bounds__(32 * (2 * R + 1), MINB) tile_stage_kernel(cons
             write_ghosts<PXY>(g, ph, a.uout, i, j, nw);
             peer_rows(a, g, i, j, nw);
         }
-        flag_nonphysical(a.st, nw);
+        flag_nonphysical(setup ? &a.st->flags0 : &a.st->nonphysical, nw);
         if (a.completes_step && a.want_cfl) lam = wave_speed(g, ph, nw);
     }
     // wave-speed max for the next step's CFL dt: one atomic per warp
