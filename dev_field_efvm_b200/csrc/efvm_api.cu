@@ -46,6 +46,10 @@ struct efvm_ctx {
     bool lam_stale = true;
     bool ghosts_stale = true;
     bool control_dirty = true;
+    // the device's step counter after the last call that read it; unknown once
+    // work was enqueued without reading it back
+    uint64_t known_step = 0;
+    bool step_known = true;
     // IBM
     bool ibm = false;
     bool geom_dirty = false;
@@ -1129,6 +1133,8 @@ int efvm_set_solver_state(efvm_ctx* c, const efvm_solver_state* in) {
     CUDA_TRY(c, cudaMemcpyAsync(c->st, &s, sizeof(DevState), cudaMemcpyHostToDevice, S(c)));
     CUDA_TRY(c, cudaStreamSynchronize(S(c)));
     c->rk_stage = in->rk_stage;
+    c->known_step = in->step;
+    c->step_known = true;
     c->lam_stale = true;
     return EFVM_OK;
 }
@@ -1410,6 +1416,7 @@ int efvm_substep(efvm_ctx* c) {
     if (!c) return fail(c, EFVM_ERR_INVALID_ARG, "null argument");
     int rc0 = finish_forces(c);
     if (rc0) return rc0;
+    c->step_known = false;
     if (c->control_dirty) sync_control(c, 0, 0.0, 0);
     int rc = prologue(c);
     if (rc) return rc;
@@ -1439,12 +1446,15 @@ int efvm_step(efvm_ctx* c, int64_t n_steps, int32_t stop_at_t, double t_stop, do
     if (c->params.integrator != EFVM_INTEGRATOR_EULER && c->rk_stage != 0)
         return fail(c, EFVM_ERR_INVALID_ARG, "efvm_step must start at a step boundary (rk_stage == 0)");
     const bool async = !stop_at_t && !force_history && !info;
-    DevState s_before{};
     int rc = EFVM_OK;
-    if (!async) {
-        rc = read_state(c, s_before);
+    if (!async && !c->step_known) {
+        DevState s;
+        rc = read_state(c, s);
         if (rc) return rc;
+        c->known_step = s.step;
     }
+    const uint64_t step_before = c->known_step;
+    c->step_known = false;
     const int subs = c->params.integrator == EFVM_INTEGRATOR_EULER ? 1 : 3;
     const long long cap = force_history && c->ibm ? (long long)subs * n_steps : 0;
     if (cap > c->history_cap) {
@@ -1457,7 +1467,9 @@ int efvm_step(efvm_ctx* c, int64_t n_steps, int32_t stop_at_t, double t_stop, do
     }
     if (c->graph_with_history != (cap != 0)) c->graph_valid = false;
     c->graph_with_history = cap != 0;
-    if (!async || c->control_dirty) {
+    // a run without a stop time and a history finds the control of such a run on the
+    // device unless the last call set another
+    if (stop_at_t || cap || c->control_dirty) {
         // forces a previous call left pending go into that call's history, not this one's
         rc = finish_forces(c);
         if (rc) return rc;
@@ -1503,8 +1515,10 @@ int efvm_step(efvm_ctx* c, int64_t n_steps, int32_t stop_at_t, double t_stop, do
                                cudaMemcpyDeviceToHost));
     else if (force_history && !c->ibm)
         std::memset(force_history, 0, (size_t)subs * n_steps * 6 * sizeof(double));
+    c->known_step = s.step;
+    c->step_known = true;
     if (info) {
-        info->steps_done = (int64_t)(s.step - s_before.step);
+        info->steps_done = (int64_t)(s.step - step_before);
         info->substeps_done = info->steps_done * subs;
         info->time = s.time;
         info->dt = s.dt;
@@ -1729,6 +1743,7 @@ int efvm_profile_steps(efvm_ctx* c, int64_t n_steps, double out_ms[4]) {
     if (!c || !out_ms || n_steps < 0) return fail(c, EFVM_ERR_INVALID_ARG, "invalid argument");
     if (c->params.integrator == EFVM_INTEGRATOR_EULER || c->rk_stage != 0)
         return fail(c, EFVM_ERR_INVALID_ARG, "efvm_profile_steps needs an RK3 context at a step boundary");
+    c->step_known = false;
     {
         const int rcf = finish_forces(c);
         if (rcf) return rcf;
@@ -1852,6 +1867,7 @@ int efvm_autotune_stage(efvm_ctx* c, int32_t n_steps, double* best_ms_per_step) 
         return fail(c, EFVM_ERR_UNSUPPORTED, "stage tuning covers 2-D RK3 contexts without slabs or a flux correction");
     if (c->rk_stage != 0) return fail(c, EFVM_ERR_INVALID_ARG, "efvm_autotune_stage needs a step boundary");
     if (n_steps <= 0) n_steps = 3;
+    c->step_known = false;
     int rc = finish_forces(c);
     if (rc) return rc;
     if (c->control_dirty) sync_control(c, 0, 0.0, 0);

@@ -132,8 +132,11 @@ def load(path: str | None = None) -> C.CDLL:
     return L
 
 
+_DP = C.POINTER(C.c_double)
+
+
 def _dp(a: np.ndarray):
-    return a.ctypes.data_as(C.POINTER(C.c_double))
+    return C.cast(a.__array_interface__["data"][0], _DP)
 
 
 class Context:
