@@ -457,6 +457,7 @@ __global__ void __launch_bounds__(128) nn_backward_kernel(PrimView pv, Net net, 
         *reinterpret_cast<uint4*>(sm + BW_ONE2 + tc::canon_offset(r, 0, 128)) = ones;
     }
     tile_setup(t, &bar, &slot, BWD_COLS);
+    pdl_wait_then_release();
     const uint32_t idesc_t = tc::idesc_bf16_f32(128, H) | tc::A_MN | tc::B_MN;
     bool ok = true, first = true;
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
@@ -549,11 +550,12 @@ __global__ void __launch_bounds__(128) nn_backward_kernel(PrimView pv, Net net, 
 // first thread also passes the loss on with the tensor-core status beside it,
 // so that the host reads both with one copy.  (One thread per parameter over
 // 2048 per-tile partials took 84 us: 19 blocks of serial loads.)
-constexpr int RED_SLICES = 8;
+constexpr int RED_SLICES = 32;
 __global__ void __launch_bounds__(32 * RED_SLICES) nn_reduce_kernel(const float* __restrict__ partials, int blocks,
                                                                     float* __restrict__ grad,
                                                                     float* __restrict__ grad_out, double* loss) {
     __shared__ float sum[RED_SLICES][32];
+    pdl_wait_then_release();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int p = blockIdx.x * 32 + lane;
     float s = 0.f;
@@ -579,6 +581,7 @@ __global__ void __launch_bounds__(256) nn_residual_kernel(const float* __restric
                                                           double inv_dx, double inv_dy, float w0, float w1, float w2,
                                                           float w3, float* __restrict__ dcorr, double* loss) {
     __shared__ double red[8];
+    pdl_wait_then_release();
     const long long n = (long long)nx * ny, total = (long long)batch * n;
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     double l = 0.0;
@@ -909,17 +912,19 @@ int efvm_nn_loss_grad(efvm_nn* h, const double* states, const double* resid, int
     nn::PackedStates sv{states, nx, ny};
     const long long cells = (long long)batch * nx * ny;
     const int tiles = (int)(2 * cells / 128);
+    NN_TRY(h, cudaMemsetAsync(h->loss_d, 0, sizeof(double), s));
     nn::nn_prims_kernel<nn::PackedStates><<<(unsigned)((cells + 255) / 256), 256, 0, s>>>(sv, batch, h->gamma, h->prims);
     const nn::PrimView pv{h->prims, nx, ny};
-    launch_forward(pv, h, tiles, h->corr, 0.f, nullptr, false, s);
-    NN_TRY(h, cudaMemsetAsync(h->loss_d, 0, sizeof(double), s));
-    nn::nn_residual_kernel<<<(unsigned)((cells + 255) / 256), 256, 0, s>>>(h->corr, resid, batch, nx, ny, 1.0 / dx,
-                                                                         1.0 / dy, w[0], w[1], w[2], w[3], h->dcorr,
-                                                                         h->loss_d);
+    // The chain is launched programmatically: each kernel sets up (weights, tensor
+    // memory) while its predecessor drains.
+    launch_forward(pv, h, tiles, h->corr, 0.f, nullptr, true, s);
     const int blocks = nn_blocks(tiles, nn::BWD_BLOCKS);
-    nn::nn_backward_kernel<<<blocks, 128, nn::SM_BWD, s>>>(pv, nn_net(h), tiles, h->dcorr, h->partials);
-    nn::nn_reduce_kernel<<<(nn::P_COUNT + 31) / 32, 32 * nn::RED_SLICES, 0, s>>>(h->partials, blocks, h->grad, grad_out,
-                                                                                 h->loss_d);
+    launch_nn(nn::nn_residual_kernel, (unsigned)((cells + 255) / 256), 256u, (size_t)0, s, true, (const float*)h->corr,
+              resid, batch, nx, ny, 1.0 / dx, 1.0 / dy, w[0], w[1], w[2], w[3], h->dcorr, h->loss_d);
+    launch_nn(nn::nn_backward_kernel, (unsigned)blocks, 128u, (size_t)nn::SM_BWD, s, true, pv, nn_net(h), tiles,
+              (const float*)h->dcorr, h->partials);
+    launch_nn(nn::nn_reduce_kernel, (unsigned)((nn::P_COUNT + 31) / 32), 32u * nn::RED_SLICES, (size_t)0, s, true,
+              (const float*)h->partials, blocks, h->grad, grad_out, h->loss_d);
     NN_TRY(h, cudaGetLastError());
     double out[2] = {0.0, 0.0};  // the loss and the tensor-core status
     NN_TRY(h, cudaMemcpyAsync(out, h->loss_d, sizeof(out), cudaMemcpyDeviceToHost, s));
