@@ -1572,10 +1572,19 @@ int launch_batch_stage(const BatchStageArgs& b, int n_tiles, bool pdl, void* str
     return 1;
 }
 
+// The persistent kernel reads each case's geometry and physics from the table, which
+// costs registers: its FP32 inviscid form spills 240 B per thread at the eight
+// blocks of the single-case form and 190 B at seven (48 cases of 32^2 to 512^2,
+// 32 steps: 11.0 -> 9.8 ms; six blocks 10.9, five 10.7).
+template <class R, bool VISC>
+static constexpr int persist_blocks() {
+    return sizeof(R) == sizeof(float) && !VISC ? 7 : StageForm<R, VISC>::MINB;
+}
+
 template <int SCHEME, int RECON, class R, bool VISC>
 static void launch_persist_f(const PersistArgs& p, int blocks, cudaStream_t s) {
     using F = StageForm<R, VISC>;
-    launch_k(batch_persistent_kernel<SCHEME, RECON, R, F::MINB, VISC, F::XFIRST>, dim3(blocks), dim3(32 * WPB), s,
+    launch_k(batch_persistent_kernel<SCHEME, RECON, R, persist_blocks<R, VISC>(), VISC, F::XFIRST>, dim3(blocks), dim3(32 * WPB), s,
              false, p);
 }
 
@@ -1599,7 +1608,10 @@ static void launch_persist_r(const PersistArgs& p, int blocks, cudaStream_t s) {
 #undef EFVM_PERSIST_V
 }
 
-int batch_form_blocks(bool fp32, bool viscous) { return form_minb(fp32, viscous); }
+int batch_form_blocks(bool fp32, bool viscous) {
+    return fp32 ? (viscous ? persist_blocks<float, true>() : persist_blocks<float, false>())
+                : (viscous ? persist_blocks<double, true>() : persist_blocks<double, false>());
+}
 
 // One block per resident slot (blocks_per_sm on every SM): the warps take their
 // work from the ticket counter, so the grid does not depend on the table.
