@@ -305,6 +305,9 @@ __global__ void __launch_bounds__(32 * WPB3, MINB3) stage3_kernel(StageArgs a, i
             zrB[1] = MUSCL && ph.periodic_z && true_seam;
         }
         const double dt = a.st->dt;
+        const bool with_u0 = a.stage == 1 || a.stage == 2;
+        const double w0 = a.stage == 1 ? 0.75 : (1.0 / 3.0), w1 = a.stage == 1 ? 0.25 : (2.0 / 3.0);
+        const bool xz_edge = i < NG || i >= g.nx - NG || k < NG || k >= g.nz - NG;  // fills ghosts in x or z
 
         V5 uc = ldrow(jb - 1), un = ldrow(jb), pc = uc;
         if (MUSCL) {
@@ -436,10 +439,12 @@ __global__ void __launch_bounds__(32 * WPB3, MINB3) stage3_kernel(StageArgs a, i
                 V5 mn;
                 slope_faces5(limiter, uc, un, un2, pn, mn);
                 const bool lo_edge = j == -1, hi_edge = j + 1 == g.ny;
-                const bool rb = lo_edge ? seam_rec_y : (hi_edge ? edge_rec_y : true);
-                const bool rt = lo_edge ? edge_rec_y : (hi_edge ? seam_rec_y : true);
-                yb_ = yq5(rb ? pc : uc);
-                yt_ = yq5(rt ? mn : un);
+                if (lo_edge || hi_edge) {
+                    if (!(lo_edge ? seam_rec_y : edge_rec_y)) pc = uc;
+                    if (!(lo_edge ? edge_rec_y : seam_rec_y)) mn = un;
+                }
+                yb_ = yq5(pc);
+                yt_ = yq5(mn);
             } else {
                 yb_ = yq5(uc);
                 yt_ = yq5(un);
@@ -453,7 +458,9 @@ __global__ void __launch_bounds__(32 * WPB3, MINB3) stage3_kernel(StageArgs a, i
                 double rhs[5];
 #pragma unroll
                 for (int v = 0; v < 5; ++v) rhs[v] = __fma_rn(-yt[v], g.inv_y, acc[v]);
-                const bool ibm = a.mask != nullptr;
+                // bodies, body force and sponge are not compiled into the periodic inviscid forms
+                constexpr bool LEAN = PXYZ;
+                const bool ibm = !LEAN && a.mask != nullptr;
                 const bool solid = ibm && a.mask[o];
                 if (VISC && !solid) {
                     // viscous_system, crates/cfd_solver/src/lib.rs:514-557 (7-point stencil),
@@ -521,16 +528,14 @@ __global__ void __launch_bounds__(32 * WPB3, MINB3) stage3_kernel(StageArgs a, i
                 if (solid)  // zero_solid_rhs, crates/cfd_ibm/src/lib.rs:293-301
 #pragma unroll
                     for (int v = 0; v < 5; ++v) rhs[v] = 0.0;
-                if (ph.body_force_x != 0.0) {  // crates/cfd_solver/tests/poiseuille_channel_validation.rs:100-118
+                if (!LEAN && ph.body_force_x != 0.0) {  // crates/cfd_solver/tests/poiseuille_channel_validation.rs:100-118
                     rhs[1] += ucd.r * ph.body_force_x;
                     rhs[4] += ph.body_force_x * ucd.mx;
                 }
                 // Rk3Integrator / EulerIntegrator::substep, crates/cfd_solver/src/integrate.rs:48-101
                 const double ucv[5] = {ucd.r, ucd.mx, ucd.my, ucd.mz, ucd.E};
                 double nwv[5];
-                if (a.stage == 1 || a.stage == 2) {
-                    const double w0 = a.stage == 1 ? 0.75 : (1.0 / 3.0);
-                    const double w1 = a.stage == 1 ? 0.25 : (2.0 / 3.0);
+                if (with_u0) {
 #pragma unroll
                     for (int v = 0; v < 5; ++v)
                         nwv[v] = __fma_rn(w1, __fma_rn(rhs[v], dt, ucv[v]), __dmul_rn(w0, a.u0[v * P + o]));
@@ -539,7 +544,7 @@ __global__ void __launch_bounds__(32 * WPB3, MINB3) stage3_kernel(StageArgs a, i
                     for (int v = 0; v < 5; ++v) nwv[v] = __fma_rn(rhs[v], dt, ucv[v]);
                 }
                 U5 nwu{nwv[0], nwv[1], nwv[2], nwv[3], nwv[4]};
-                if (a.completes_step && ph.sponge) {
+                if (!LEAN && a.completes_step && ph.sponge) {
                     // the sphere case's outlet sponge toward the uniform freestream
                     // (rho, u_max, 0, 0, p), examples/sphere_drag_validation/main.rs:119-160
                     const double cx = centre(g.lo[0], g.h[0], i);
@@ -556,13 +561,16 @@ __global__ void __launch_bounds__(32 * WPB3, MINB3) stage3_kernel(StageArgs a, i
                     }
                 }
                 store5(a.uout, P, o, nwu);
-                write_ghosts3<PXYZ>(g, ph, a.uout, i, j, k, nwu);
+                if (xz_edge || j < NG || j >= g.ny - NG) write_ghosts3<PXYZ>(g, ph, a.uout, i, j, k, nwu);
+                // a NaN in any component fails one of the two tests
                 int bad = 0;
                 if (!(nwu.r > 0.0)) bad |= 1;
                 if (!(2.0 * nwu.E * nwu.r > nwu.mx * nwu.mx + nwu.my * nwu.my + nwu.mz * nwu.mz)) bad |= 2;
-                if (nwu.r != nwu.r || nwu.mx != nwu.mx || nwu.my != nwu.my || nwu.mz != nwu.mz || nwu.E != nwu.E)
-                    bad |= 4;
-                if (bad) atomicOr(&a.st->nonphysical, bad);
+                if (bad) {
+                    if (nwu.r != nwu.r || nwu.mx != nwu.mx || nwu.my != nwu.my || nwu.mz != nwu.mz || nwu.E != nwu.E)
+                        bad |= 4;
+                    atomicOr(&a.st->nonphysical, bad);
+                }
                 if (a.completes_step && a.want_cfl) lam = fmax(lam, wave_speed3(g, ph, nwu));
             }
             gb = gt;
@@ -897,7 +905,8 @@ static void launch_stage3_t(const StageArgs& a, bool pdl, cudaStream_t s) {
     if constexpr (VISC) {
         launch_stage3_k<SCHEME, RECON, VISC, -1, false>(a, pdl, s);
     } else {
-        const bool pxyz = a.ph.periodic_x && a.ph.periodic_y && a.ph.periodic_z;
+        const bool pxyz = a.ph.periodic_x && a.ph.periodic_y && a.ph.periodic_z && a.mask == nullptr && !a.ph.sponge &&
+                          a.ph.body_force_x == 0.0;
         if constexpr (RECON == EFVM_RECON_MUSCL) {
             if (a.ph.limiter == EFVM_LIMITER_MC)
                 pxyz ? launch_stage3_k<SCHEME, RECON, VISC, EFVM_LIMITER_MC, true>(a, pdl, s)
