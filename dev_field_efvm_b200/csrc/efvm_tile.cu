@@ -20,9 +20,11 @@
 // one copy of the flux code; the price is (R + 1) / R y faces per row and a memory
 // latency and a barrier per tile, which lose to the TMA-fed form where the grid
 // is many waves of tiles.  us per step, strip or TMA form -> this kernel:
-// vortex 64^2 22.6 -> 13.2, 128^2 26.1 -> 16.2, 512^2 77 -> 53, 1024^2 193 -> 186,
-// 2048^2 504 -> 715; cylinder 440x82 first order 43.1 -> 30.7, 1100x205 MUSCL 77.8
-// -> 68.8, 2200x410 203 -> 203.
+// vortex 64^2 22.6 -> 12.3, 128^2 24.4 -> 14.4, 512^2 57.5 -> 53.9, 768^2 95.7 -> 106;
+// cylinder 440x82 first order 42.5 -> 26.7, 1100x205 MUSCL 77.7 -> 68.5, 2200x410
+// 203 -> 203.  (Persistent blocks with double-buffered TMA tiles measured 18.5 us at
+// 128^2, 69.5 at 1100x205 and 129 at 1003x777, and won only on large viscous grids,
+// 4400x820 744 -> 709: dropped.)
 //
 // R = 3 rows and four resident blocks (28 warps per SM, 72 registers) measured
 // fastest over 128^2 to 1100x205 among R = 2 .. 7 and 18 to 30 warps: 1100x205

@@ -354,8 +354,8 @@ int efvm_profile_steps(efvm_ctx* ctx, int64_t n_steps, double out_ms[4]);
  * the strip form whatever is set.
  * EFVM_STAGE_AUTO is the built-in choice: the TMA-fed form wherever the case
  * allows it (the faster of the two at 4096^2 in both precisions), else the
- * strip form; an FP64 case of up to 800,000 cells without explicit rows or
- * blocks runs a build of the strip form with one face per lane (reported by
+ * strip form; an FP64 case of up to 400,000 cells (800,000 where the TMA-fed
+ * form does not run) without explicit rows or blocks runs a build of the strip form with one face per lane (reported by
  * efvm_get_stage_tiling as the strip form).  Both give the reference's results
  * (the forms, and the strip form's builds for different block counts, differ
  * from each other by a few ulps at most; a form gives the same bits for any
