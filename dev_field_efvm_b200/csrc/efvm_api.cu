@@ -68,6 +68,7 @@ struct efvm_ctx {
     efvm_nn* nn = nullptr;
     float* corr = nullptr;               // [2][4][ny][nx]
     float4* prims = nullptr;             // the network's per-cell inputs
+    bool prims_stale = true;             // not those of the current state (fused_prims)
     unsigned long long* fallbacks = nullptr;
     float sensor = 0.f;
     uint64_t corr_faces = 0;
@@ -487,6 +488,25 @@ int build_ibm_lists3(efvm_ctx* c) {
     return EFVM_OK;
 }
 
+// Whether the built-in choice is the face-parallel kernel (efvm_tile.cu): an FP64
+// case without explicit form, rows and blocks, up to a number of cells.  The lines
+// lie where the forms measured equal (us per step, other form / face-parallel):
+// against the TMA-fed form 512^2 57.5 / 53.9, 768^2 95.7 / 106, 1003x777 121 / 140;
+// against the viscous strip form 1500x279 113 / 105, 2200x410 203 / 203.
+constexpr long long TILE_CELLS_TMA = 400000, TILE_CELLS_STRIP = 800000;
+bool use_tile(const efvm_ctx* c) {
+    if (c->g.nz > 1 || c->ph.precision != EFVM_PREC_FP64 || c->stage_form != EFVM_STAGE_AUTO || c->stage_rows != 0 ||
+        c->stage_blocks != 0)
+        return false;
+    const bool tma = c->tmaps && stage_tma_eligible(c->g, c->ph, c->ibm, c->nn != nullptr);
+    return (long long)c->g.nx * c->g.ny <= (tma ? TILE_CELLS_TMA : TILE_CELLS_STRIP);
+}
+
+// With corrections the face-parallel stages leave the network's inputs of their
+// output in c->prims, so the next stage needs no pass over the state; any other
+// form of the stage, and whatever replaces the state, makes them stale.
+bool fused_prims(const efvm_ctx* c) { return c->nn && use_tile(c); }
+
 // Setup-phase work that precedes a step boundary's first stage, in the
 // reference's Setup order: CFL (SolverPlugin) before the geometry refresh
 // (CylinderIbmPlugin), then Halo/Boundary for a state that changed on the host.
@@ -515,6 +535,12 @@ int prologue(efvm_ctx* c) {
         c->launches += launch_fill_ghosts(c->g, c->ph, cur_buf(c), S(c));
         c->ghosts_stale = false;
     }
+    if (c->nn) {
+        if (fused_prims(c) && c->prims_stale)
+            c->launches += nn_prims_padded(c->nn, cur_buf(c), c->g.plane, c->g.pitch, c->g.nx, c->g.ny, c->prims, S(c));
+        // what follows the prologue is a stage, which leaves them fresh or not by its form
+        c->prims_stale = !fused_prims(c);
+    }
     return EFVM_OK;
 }
 
@@ -529,27 +555,17 @@ int resolved_form(const efvm_ctx* c) {
     return EFVM_STAGE_STRIP;
 }
 
-// Whether the built-in choice is the face-parallel kernel (efvm_tile.cu): an FP64
-// case without explicit form, rows and blocks, up to a number of cells.  The lines
-// lie where the forms measured equal (us per step, other form / face-parallel):
-// against the TMA-fed form 512^2 57.5 / 53.9, 768^2 95.7 / 106, 1003x777 121 / 140;
-// against the viscous strip form 1500x279 113 / 105, 2200x410 203 / 203.
-constexpr long long TILE_CELLS_TMA = 400000, TILE_CELLS_STRIP = 800000;
-bool use_tile(const efvm_ctx* c) {
-    if (c->g.nz > 1 || c->ph.precision != EFVM_PREC_FP64 || c->stage_form != EFVM_STAGE_AUTO || c->stage_rows != 0 ||
-        c->stage_blocks != 0)
-        return false;
-    const bool tma = c->tmaps && stage_tma_eligible(c->g, c->ph, c->ibm, c->nn != nullptr);
-    return (long long)c->g.nx * c->g.ny <= (tma ? TILE_CELLS_TMA : TILE_CELLS_STRIP);
-}
-
 void enqueue_stage_kernel(efvm_ctx* c, int stage, double* uin, double* uout, bool pdl = true, bool defer = false,
                           bool fold_setup = false) {
-    if (c->nn)  // the learned corrections of this stage's input
+    if (c->nn && fused_prims(c))  // the learned corrections of this stage's input
+        c->launches += nn_forward_prims(c->nn, c->g.nx, c->g.ny, c->corr, c->prims, c->sensor, c->fallbacks, S(c));
+    else if (c->nn)
         c->launches += nn_forward_padded(c->nn, uin, c->g.plane, c->g.pitch, c->g.nx, c->g.ny, c->corr, c->prims,
                                          c->sensor, c->fallbacks, S(c));
     StageArgs a{};
     a.corr = c->nn ? c->corr : nullptr;
+    a.prims = c->prims;
+    a.prim_gamma = c->nn ? nn_gamma(c->nn) : 0.f;
     a.g = c->g;
     a.ph = c->ph;
     a.uin = uin;
@@ -1034,6 +1050,7 @@ static int transfer_state(efvm_ctx* c, double* base, int64_t si, int64_t sj, int
         CUDA_TRY(c, cudaMemcpyAsync(c->staging, host0, (size_t)span * sizeof(double), cudaMemcpyHostToDevice, S(c)));
         c->launches += launch_pack(g, dev0, si, sj, sv, q, 1, S(c));
         c->lam_stale = true;
+        c->prims_stale = true;
         c->ghosts_stale = true;
     } else {
         if (!dense)  // keep the caller's values in the gaps of a sparse layout
@@ -1140,6 +1157,7 @@ int efvm_set_solver_state(efvm_ctx* c, const efvm_solver_state* in) {
     c->known_step = in->step;
     c->step_known = true;
     c->lam_stale = true;
+    c->prims_stale = true;  // another RK stage is another buffer
     return EFVM_OK;
 }
 
@@ -1165,6 +1183,7 @@ int efvm_set_flux_correction(efvm_ctx* c, efvm_nn* nn, float sensor) {
     CUDA_TRY(c, cudaMemsetAsync(c->fallbacks, 0, sizeof(unsigned long long), S(c)));
     if (nn_prepare_launches()) return fail(c, EFVM_ERR_CUDA, "flux correction: kernel attributes");
     c->nn = nn;
+    c->prims_stale = true;
     c->sensor = sensor;
     c->corr_faces = 0;
     c->graph_valid = false;
@@ -1720,6 +1739,7 @@ int efvm_init_vortex(efvm_ctx* c, const efvm_vortex* v) {
     }
     c->launches += launch_init_vortex(c->g, *v, cur_buf(c), S(c));
     c->lam_stale = true;
+    c->prims_stale = true;
     c->ghosts_stale = true;
     CUDA_TRY(c, cudaStreamSynchronize(S(c)));
     return EFVM_OK;

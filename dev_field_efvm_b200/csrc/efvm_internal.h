@@ -13,6 +13,8 @@
 // (efvm_kernels3d.cuh).
 #pragma once
 
+#include <cuda_runtime.h>
+
 #include <cstdint>
 #include <string>
 #include <vector>
@@ -201,6 +203,8 @@ struct StageArgs {
     int completes_step;               // sponge + CFL + clock in the epilogue
     int want_cfl;
     const float* corr;                // learned face-flux corrections [2][4][ny][nx] or null
+    float4* prims;                    // face-parallel kernel with corrections: the network's inputs of the
+    float prim_gamma;                 // output, [ny][nx] (rho - 1, u, v, p - 1), with the network's gamma
     int defer_forces;                 // stage 2 of the step graph: its IBM forces run in the next launch
     // The TMA-fed stage kernel (2-D, inviscid, no bodies, no correction): host
     // copies of the tensor maps (CUtensorMap, 128 bytes) of the stage input and
@@ -297,8 +301,15 @@ int launch_clock(unsigned long long* out, void* stream);
 
 // The learned correction (efvm_nn.cu): corrections of every face of one
 // periodic context state, and the kernel attributes its launches need.
+// nn_forward_padded runs nn_prims_padded (the per-cell inputs of a state) and
+// nn_forward_prims (the corrections from them); programmatic launches.
+int nn_prims_padded(const efvm_nn* h, const double* q, long long plane, int pitch, int nx, int ny, float4* prims,
+                    void* stream);
+int nn_forward_prims(const efvm_nn* h, int nx, int ny, float* corr, float4* prims, float sensor,
+                     unsigned long long* fallbacks, void* stream);
 int nn_forward_padded(const efvm_nn* h, const double* q, long long plane, int pitch, int nx, int ny, float* corr,
                       float4* prims, float sensor, unsigned long long* fallbacks, void* stream);
+float nn_gamma(const efvm_nn* h);
 int nn_prepare_launches();
 
 // Validation and the device description of one case (efvm_api.cu): global rows

@@ -707,15 +707,28 @@ static void launch_forward(const nn::PrimView& pv, const efvm_nn* h, int tiles, 
 
 // Both launches belong to a captured step: programmatic, like its other kernels
 // (the weights do not change while a step runs).
+int nn_prims_padded(const efvm_nn* h, const double* q, long long plane, int pitch, int nx, int ny, float4* prims,
+                    void* stream) {
+    nn::PaddedState sv{q, plane, pitch, nx, ny};
+    launch_nn(nn::nn_prims_kernel<nn::PaddedState>, (unsigned)((nx * ny + 255) / 256), 256u, (size_t)0,
+              (cudaStream_t)stream, true, sv, 1, h->gamma, prims);
+    return 1;
+}
+
+int nn_forward_prims(const efvm_nn* h, int nx, int ny, float* corr, float4* prims, float sensor,
+                     unsigned long long* fallbacks, void* stream) {
+    launch_forward(nn::PrimView{prims, nx, ny}, h, (int)(2LL * nx * ny / 128), corr, sensor, fallbacks, true,
+                   (cudaStream_t)stream);
+    return 1;
+}
+
 int nn_forward_padded(const efvm_nn* h, const double* q, long long plane, int pitch, int nx, int ny, float* corr,
                       float4* prims, float sensor, unsigned long long* fallbacks, void* stream) {
-    cudaStream_t s = (cudaStream_t)stream;
-    nn::PaddedState sv{q, plane, pitch, nx, ny};
-    launch_nn(nn::nn_prims_kernel<nn::PaddedState>, (unsigned)((nx * ny + 255) / 256), 256u, (size_t)0, s, true, sv, 1,
-              h->gamma, prims);
-    launch_forward(nn::PrimView{prims, nx, ny}, h, (int)(2LL * nx * ny / 128), corr, sensor, fallbacks, true, s);
-    return 2;
+    return nn_prims_padded(h, q, plane, pitch, nx, ny, prims, stream) +
+           nn_forward_prims(h, nx, ny, corr, prims, sensor, fallbacks, stream);
 }
+
+float nn_gamma(const efvm_nn* h) { return h->gamma; }
 
 int nn_prepare_launches() {
     cudaError_t e = cudaFuncSetAttribute(nn::nn_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, nn::SM_FWD);

@@ -273,6 +273,13 @@ __global__ void __launch_bounds__(32 * (2 * R + 1), MINB) tile_stage_kernel(cons
         }
         U4 nw{un[0], un[1], un[2], un[3]};
         if (FULL && a.completes_step && ph.sponge) sponge_2d(g, ph, i, j, dt, nw);
+        if constexpr (CORR) {
+            // the network's inputs of this cell for the next stage (nn_prims_kernel forms
+            // them only after the state was replaced): a launch less per stage
+            const double pu = nw.mx / nw.r, pv = nw.my / nw.r;
+            const double pp = (a.prim_gamma - 1.0) * (nw.E - 0.5 * nw.r * (pu * pu + pv * pv));
+            a.prims[(long long)j * g.nx + i] = make_float4((float)nw.r - 1.0f, (float)pu, (float)pv, (float)pp - 1.0f);
+        }
         store4(a.uout, P, o, nw);
         if (i < NG || i >= g.nx - NG || j < NG || j >= g.ny - NG) {
             write_ghosts<PXY>(g, ph, a.uout, i, j, nw);
