@@ -424,9 +424,50 @@ __global__ void __launch_bounds__(128) nn_forward_kernel(PrimView pv, Net net, i
     tile_teardown(t, FWD_COLS);
 }
 
-// Backward: given dL/dcorr (grid frame, the layout of corr), the gradient of the
-// loss with respect to every parameter, summed over the block's tiles, into
-// partials[block][P_COUNT].
+// The residual loss of a batch: e = R + div(corr) per cell and variable,
+// L = sum_v w_v mean(e_v^2).
+struct Residual {
+    const float* corr;    // the forward pass's corrections, grid frame
+    const double* resid;  // R, [batch][4][ny][nx]
+    double inv_dx, inv_dy;
+    float w[4];
+    double inv_cells;     // 1 / (batch ny nx)
+    double* loss;
+};
+
+// dL/dcorr of one face in the grid frame, from the errors of the two cells it
+// divides (+1/dx in the cell before it, -1/dx in its own), and for an x face the
+// loss of its own cell, added to `l`.
+__device__ __forceinline__ void face_gradient(const Residual& rs, const FaceId& id, int nx, int ny, float (&g)[4],
+                                              double& l) {
+    const long long n = (long long)nx * ny;
+    const int i = id.i, j = id.j;
+    const int im = i == 0 ? nx - 1 : i - 1, ip = i == nx - 1 ? 0 : i + 1;
+    const int jm = j == 0 ? ny - 1 : j - 1, jp = j == ny - 1 ? 0 : j + 1;
+    const bool x = id.orient == 0;
+    // the other cell of the face, and the cells after it
+    const int oi = x ? im : i, oj = x ? j : jm;
+    const int oip = x ? i : ip, ojp = x ? jp : j;
+    const int c = j * nx + i, o = oj * nx + oi;
+    const double inv = x ? rs.inv_dx : rs.inv_dy;
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+        const float* cx = rs.corr + ((long long)(id.b * 2 + 0) * 4 + v) * n;  // x face on the left of a cell
+        const float* cy = rs.corr + ((long long)(id.b * 2 + 1) * 4 + v) * n;  // y face below it
+        const double* r = rs.resid + ((long long)id.b * 4 + v) * n;
+        auto err = [&](int cell, int right, int above) {
+            return r[cell] + (((double)cx[right] - (double)cx[cell]) * rs.inv_dx +
+                              ((double)cy[above] - (double)cy[cell]) * rs.inv_dy);
+        };
+        const double e = err(c, j * nx + ip, jp * nx + i), eo = err(o, oj * nx + oip, ojp * nx + oi);
+        if (x) l += rs.w[v] * e * e;
+        g[v] = (float)(2.0 * rs.inv_cells * rs.w[v] * (eo - e) * inv);
+    }
+}
+
+// Backward: the loss, and its gradient with respect to every parameter summed over
+// the block's tiles, into partials[block][P_COUNT].  Each face forms its own dL/dcorr
+// (a kernel of its own took 8 us at 131072 cells, and 4 MB out and back).
 //
 // Per tile four product phases form the chain: X W1^T; H1 W2^T; dZ2 W2 (beside
 // dW3 += H2^T dY and dW2 += H1^T dZ2); dW1 += X^T dZ1.  The weight gradients
@@ -436,8 +477,7 @@ __global__ void __launch_bounds__(128) nn_forward_kernel(PrimView pv, Net net, i
 // the FP32 units.  One block per tile with stored transposes (150 KB, one block
 // per SM), shuffled column sums for the biases and 39 MB of per-tile partials
 // took 235 us and 84 us for their sum at 262144 faces.
-__global__ void __launch_bounds__(128) nn_backward_kernel(PrimView pv, Net net, int tiles,
-                                                          const float* __restrict__ dcorr,
+__global__ void __launch_bounds__(128) nn_backward_kernel(PrimView pv, Net net, int tiles, Residual rs,
                                                           float* __restrict__ partials) {
     extern __shared__ __align__(128) unsigned char sm[];
     __shared__ __align__(8) uint64_t bar;
@@ -460,13 +500,12 @@ __global__ void __launch_bounds__(128) nn_backward_kernel(PrimView pv, Net net, 
     pdl_wait_then_release();
     const uint32_t idesc_t = tc::idesc_bf16_f32(128, H) | tc::A_MN | tc::B_MN;
     bool ok = true, first = true;
+    double l = 0.0;
     for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         const FaceId id = face_of((long long)tile * 128 + r, pv.nx, pv.ny);
         // output gradient of this face in its own frame, times out_scale, as BF16
-        const long long cell = (long long)id.j * pv.nx + id.i, nn = (long long)pv.nx * pv.ny;
         float g[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) g[q] = dcorr[((long long)(id.b * 2 + id.orient) * 4 + q) * nn + cell];
+        face_gradient(rs, id, pv.nx, pv.ny, g, l);
         const float dyf[4] = {g[0] * net.out_scale, (id.orient == 0 ? g[1] : g[2]) * net.out_scale,
                               (id.orient == 0 ? g[2] : g[1]) * net.out_scale, g[3] * net.out_scale};
         float dy[4];
@@ -515,6 +554,8 @@ __global__ void __launch_bounds__(128) nn_backward_kernel(PrimView pv, Net net, 
         first = false;
         if (!(ok = products_done(t))) break;
     }
+    for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+    if ((r & 31) == 0 && l != 0.0) atomicAdd(rs.loss, l * rs.inv_cells);
     if (ok) {
         // row k of the transposed gradients is feature k; the row of ones holds the biases
         float* part = partials + (long long)blockIdx.x * P_COUNT;
@@ -572,54 +613,6 @@ __global__ void __launch_bounds__(32 * RED_SLICES) nn_reduce_kernel(const float*
     if (blockIdx.x == 0 && threadIdx.x == 0) loss[1] = (double)g_nn_error;
 }
 
-// Residual loss of a batch: e = R + div(corr) per cell and variable,
-// L = sum_v w_v * mean(e_v^2); dcorr = dL/dcorr.  One thread per cell; the
-// loss goes out with one atomic per block (one per warp serialised on the one
-// address: 13.4 us at 131072 cells).
-__global__ void __launch_bounds__(256) nn_residual_kernel(const float* __restrict__ corr,
-                                                          const double* __restrict__ resid, int batch, int nx, int ny,
-                                                          double inv_dx, double inv_dy, float w0, float w1, float w2,
-                                                          float w3, float* __restrict__ dcorr, double* loss) {
-    __shared__ double red[8];
-    pdl_wait_then_release();
-    const long long n = (long long)nx * ny, total = (long long)batch * n;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    double l = 0.0;
-    if (t < total) {
-        const int b = (int)(t / n);
-        const int cell = (int)(t - (long long)b * n);
-        const int j = cell / nx, i = cell - j * nx;
-        const int im = i == 0 ? nx - 1 : i - 1, ip = i == nx - 1 ? 0 : i + 1;
-        const int jr = j * nx, jm = (j == 0 ? ny - 1 : j - 1) * nx, jp = (j == ny - 1 ? 0 : j + 1) * nx;
-        const float w[4] = {w0, w1, w2, w3};
-        const double scale = 2.0 / (double)total;
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            const float* cx = corr + ((long long)(b * 2 + 0) * 4 + v) * n;  // x face on the left of a cell
-            const float* cy = corr + ((long long)(b * 2 + 1) * 4 + v) * n;  // y face below it
-            const double* rs = resid + ((long long)b * 4 + v) * n;
-            const double x0 = cx[jr + i], y0 = cy[jr + i];
-            auto err = [&](double r, double xr, double xl, double yt, double yb) {
-                return r + ((xr - xl) * inv_dx + (yt - yb) * inv_dy);
-            };
-            const double e = err(rs[jr + i], cx[jr + ip], x0, cy[jp + i], y0);
-            const double ex = err(rs[jr + im], x0, cx[jr + im], cy[jp + im], cy[jr + im]);
-            const double ey = err(rs[jm + i], cx[jm + ip], cx[jm + i], y0, cy[jm + i]);
-            l += w[v] * e * e;
-            // x face on the left of (i, j): +1/dx in cell (i-1, j), -1/dx in cell (i, j)
-            dcorr[((long long)(b * 2 + 0) * 4 + v) * n + cell] = (float)(scale * w[v] * (ex - e) * inv_dx);
-            dcorr[((long long)(b * 2 + 1) * 4 + v) * n + cell] = (float)(scale * w[v] * (ey - e) * inv_dy);
-        }
-    }
-    for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = l;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int k = 1; k < 8; ++k) l += red[k];
-        if (l != 0.0) atomicAdd(loss, l / (double)total);
-    }
-}
-
 // Adam on the FP32 parameters, then the BF16 copies the tensor cores read.
 __global__ void nn_adam_kernel(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v,
                                const float* __restrict__ g, float lr, float b1t, float b2t,
@@ -655,7 +648,7 @@ struct efvm_nn {
     int64_t steps = 0;
     float* partials = nullptr;
     size_t partials_cap = 0;
-    float *corr = nullptr, *dcorr = nullptr;
+    float* corr = nullptr;
     size_t corr_cap = 0;
     float4* prims = nullptr;
     size_t prims_cap = 0;
@@ -802,11 +795,9 @@ int ensure_buffers(efvm_nn* h, int batch, int nx, int ny) {
     }
     if (faces * 4 > h->corr_cap) {
         cudaFree(h->corr);
-        cudaFree(h->dcorr);
-        h->corr = h->dcorr = nullptr;
+        h->corr = nullptr;
         h->corr_cap = 0;
         NN_TRY(h, cudaMalloc(&h->corr, faces * 4 * sizeof(float)));
-        NN_TRY(h, cudaMalloc(&h->dcorr, faces * 4 * sizeof(float)));
         h->corr_cap = faces * 4;
     }
     return EFVM_OK;
@@ -872,7 +863,6 @@ int efvm_nn_destroy(efvm_nn* h) {
     cudaFree(h->w3);
     cudaFree(h->partials);
     cudaFree(h->corr);
-    cudaFree(h->dcorr);
     cudaFree(h->prims);
     cudaFree(h->loss_d);
     delete h;
@@ -932,10 +922,9 @@ int efvm_nn_loss_grad(efvm_nn* h, const double* states, const double* resid, int
     // memory) while its predecessor drains.
     launch_forward(pv, h, tiles, h->corr, 0.f, nullptr, true, s);
     const int blocks = nn_blocks(tiles, nn::BWD_BLOCKS);
-    launch_nn(nn::nn_residual_kernel, (unsigned)((cells + 255) / 256), 256u, (size_t)0, s, true, (const float*)h->corr,
-              resid, batch, nx, ny, 1.0 / dx, 1.0 / dy, w[0], w[1], w[2], w[3], h->dcorr, h->loss_d);
-    launch_nn(nn::nn_backward_kernel, (unsigned)blocks, 128u, (size_t)nn::SM_BWD, s, true, pv, nn_net(h), tiles,
-              (const float*)h->dcorr, h->partials);
+    const nn::Residual rs{h->corr, resid, 1.0 / dx, 1.0 / dy, {w[0], w[1], w[2], w[3]}, 1.0 / (double)cells, h->loss_d};
+    launch_nn(nn::nn_backward_kernel, (unsigned)blocks, 128u, (size_t)nn::SM_BWD, s, true, pv, nn_net(h), tiles, rs,
+              h->partials);
     launch_nn(nn::nn_reduce_kernel, (unsigned)((nn::P_COUNT + 31) / 32), 32u * nn::RED_SLICES, (size_t)0, s, true,
               (const float*)h->partials, blocks, h->grad, grad_out, h->loss_d);
     NN_TRY(h, cudaGetLastError());
