@@ -378,7 +378,8 @@ __device__ __forceinline__ void tile_teardown(const TC& t, uint32_t cols) {
 // Bound by the latency of a tile's chain (gather 25 cells, three products and
 // their read-backs), so the blocks are persistent (weights and tensor memory
 // set up once) and small enough for five per SM, whose tiles overlap.  One
-// 87 KB block per tile, two resident, took 51 us for 262144 faces (2048 tiles).
+// 87 KB block per tile, two resident, took 51 us for 262144 faces (2048 tiles);
+// this form takes 23.5 us.
 __global__ void __launch_bounds__(128) nn_forward_kernel(PrimView pv, Net net, int tiles, float* __restrict__ corr,
                                                          float sensor, unsigned long long* fallbacks) {
     extern __shared__ __align__(128) unsigned char sm[];
@@ -476,7 +477,8 @@ __device__ __forceinline__ void face_gradient(const Residual& rs, const FaceId& 
 // so nothing is stored twice or transposed.  dH2 = dY W3 has K = 4 and runs on
 // the FP32 units.  One block per tile with stored transposes (150 KB, one block
 // per SM), shuffled column sums for the biases and 39 MB of per-tile partials
-// took 235 us and 84 us for their sum at 262144 faces.
+// took 235 us and 84 us for their sum at 262144 faces; now 43.5 and 8.9 us, the
+// residual's gradient included.
 __global__ void __launch_bounds__(128) nn_backward_kernel(PrimView pv, Net net, int tiles, Residual rs,
                                                           float* __restrict__ partials) {
     extern __shared__ __align__(128) unsigned char sm[];
@@ -590,7 +592,8 @@ __global__ void __launch_bounds__(128) nn_backward_kernel(PrimView pv, Net net, 
 // slice of the blocks over 32 parameters, then the slices in order.  The grid's
 // first thread also passes the loss on with the tensor-core status beside it,
 // so that the host reads both with one copy.  (One thread per parameter over
-// 2048 per-tile partials took 84 us: 19 blocks of serial loads.)
+// 2048 per-tile partials took 84 us: 19 blocks of serial loads; this takes 8.9 us
+// for 444.)
 constexpr int RED_SLICES = 32;
 __global__ void __launch_bounds__(32 * RED_SLICES) nn_reduce_kernel(const float* __restrict__ partials, int blocks,
                                                                     float* __restrict__ grad,

@@ -1,9 +1,9 @@
-"""The face-parallel stage kernel (the built-in choice of FP64 cases up to 800,000
-cells) against the strip kernel on the same states.  Inviscid: both evaluate the
-same explicitly rounded operations, so they agree bit for bit, whatever the
-grid's remainder against the 31 x 3 tile.  Viscous: the stencil's reciprocals are
-formed per cell instead of shared, a few ulps: 1e-13 of each variable's scale per
-step."""
+"""The face-parallel stage kernel (the built-in choice of the smaller FP64 cases: up
+to 400,000 cells where the TMA-fed form applies, 800,000 elsewhere) against the strip
+kernel on the same states.  Inviscid: both evaluate the same explicitly rounded
+operations, so they agree bit for bit, whatever the grid's remainder against the
+31 x 3 tile.  Viscous: the stencil's reciprocals are formed per cell instead of
+shared, a few ulps: 1e-13 of each variable's scale per step."""
 from __future__ import annotations
 
 import numpy as np
