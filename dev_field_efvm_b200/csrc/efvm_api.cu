@@ -489,17 +489,13 @@ int build_ibm_lists3(efvm_ctx* c) {
 }
 
 // Whether the built-in choice is the face-parallel kernel (efvm_tile.cu): an FP64
-// case without explicit form, rows and blocks, up to a number of cells.  The lines
-// lie where the forms measured equal (us per step, other form / face-parallel):
-// against the TMA-fed form 512^2 57.5 / 53.9, 768^2 95.7 / 106, 1003x777 121 / 140;
-// against the viscous strip form 1500x279 113 / 105, 2200x410 203 / 203.
-constexpr long long TILE_CELLS_TMA = 400000, TILE_CELLS_STRIP = 800000;
+// case without explicit form, rows and blocks, within the limits of tile_fits.
 bool use_tile(const efvm_ctx* c) {
     if (c->g.nz > 1 || c->ph.precision != EFVM_PREC_FP64 || c->stage_form != EFVM_STAGE_AUTO || c->stage_rows != 0 ||
         c->stage_blocks != 0)
         return false;
     const bool tma = c->tmaps && stage_tma_eligible(c->g, c->ph, c->ibm, c->nn != nullptr);
-    return (long long)c->g.nx * c->g.ny <= (tma ? TILE_CELLS_TMA : TILE_CELLS_STRIP);
+    return tile_fits((long long)c->g.nx * c->g.ny, c->g.ny, tma);
 }
 
 // With corrections the face-parallel stages leave the network's inputs of their

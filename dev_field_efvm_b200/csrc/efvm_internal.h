@@ -20,6 +20,7 @@
 #include <vector>
 
 #include "../../include/efvm.h"
+#include "efvm_plan.h"
 
 namespace efvm {
 
@@ -291,7 +292,7 @@ bool stage_tma_eligible(const Geometry& g, const Physics& ph, bool ibm, bool cor
 int encode_state_map(const Geometry& g, const double* buf, bool u0, void* map_out);
 // The face-parallel stage kernel (efvm_tile.cu): 2-D FP64 cases, tiles of
 // 31 columns x TILE_ROWS rows, TILE_BLOCKS resident blocks per SM.
-constexpr int TILE_ROWS = 3, TILE_BLOCKS = 4;
+constexpr int TILE_BLOCKS = 4;
 int launch_stage_tile(const StageArgs& a, bool pdl, void* stream);
 int launch_batch_stage(const BatchStageArgs& b, int n_tiles, bool pdl, void* stream);
 // Per-step set-up of every case (one thread each).

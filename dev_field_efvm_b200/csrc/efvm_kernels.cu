@@ -1303,33 +1303,6 @@ static int form_minb(bool fp32, bool viscous) {
                 : (viscous ? StageForm<double, true>::MINB : StageForm<double, false>::MINB);
 }
 
-// Rows each warp marches: the count in [lo, hi] whose blocks, dealt to the resident
-// slots in order, finish first.  A block of r rows takes r passes, one more that
-// only forms the face below its first row (about half a pass), and the column's
-// last block is shorter.  A count that leaves a few full blocks for one more wave
-// pays for nearly two: by the fewest-rows rule that this one replaces 1024^2 took
-// 12 rows and 1.05 waves (us per step 193 -> 159), 4400x820 viscous 804 -> 742.
-// In 3-D short last blocks fill the gaps the long ones leave (tail_cost 0.15:
-// over nine cases of 50 to 256 cells a side the choice is within 0.9 % of the best
-// of 2..16 rows on average, 3 % at most; without it 1.7 and 6 %); in 2-D the same
-// term made 1024^2 5 % and 4096^2 3 % slower.
-static int pick_rows(long long across, int ny, long long slots, int lo, int hi, double tail_cost) {
-    int best = lo;
-    double best_cost = 1e300;
-    for (int rows = lo; rows <= hi; ++rows) {
-        const int down = (ny + rows - 1) / rows, tail = ny - (down - 1) * rows;
-        const long long blocks = across * down, full = blocks / slots, over = blocks - full * slots;
-        const double last = over == 0 ? 0.0 : (over <= across ? tail + 0.5 : rows + 0.5);
-        const double cost = (double)full * (rows + 0.5) + last + tail_cost * (tail + 0.5);
-        if (cost < best_cost) {
-            best_cost = cost;
-            best = rows;
-        }
-        if (rows >= ny) break;
-    }
-    return best;
-}
-
 // Large 2-D grids take 16 rows, measured fastest at 4096^2 (ms per step, FP64
 // TMA-fed form: 8 rows 2.04, 16 rows 1.97, 32 rows 1.98).
 static int rows_per_warp(int nx, int ny, int blocks_per_sm) {

@@ -1,0 +1,80 @@
+"""The rules that lay out a stage kernel's launch (csrc/efvm_plan.h), compiled and
+run on the host: a column of blocks fits the 65,535 blocks that a launch takes
+along y for every height that the rows allow, and no grid whose column of
+face-parallel tiles does not fit is sent to that kernel."""
+from __future__ import annotations
+
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+SOURCE = r"""
+#include <cstdio>
+#include "efvm_plan.h"
+using namespace efvm;
+int main() {
+    // 2-D: one block of strips across, each resident-block count, rows in [2, 16]
+    for (int per_sm = 5; per_sm <= 8; ++per_sm)
+        for (int ny = 1; ny <= 16 * GRID_Y_MAX; ny += ny < 800000 ? 97 : 1) {
+            const int r = pick_rows(1, ny, 148LL * per_sm, 2, 16, 0.0);
+            if (r < 2 || r > 16 || (ny + r - 1) / r > GRID_Y_MAX) return std::printf("2-D %d %d %d\n", per_sm, ny, r), 1;
+        }
+    for (int across = 1; across <= 8; ++across)  // 3-D, rows in [2, 16]
+        for (int ny = 1; ny <= 16 * GRID_Y_MAX; ny += ny < 600000 ? 97 : 7) {
+            const int r = pick_rows(across, ny, 592, 2, 16, 0.15);
+            if (r < 2 || r > 16 || (ny + r - 1) / r > GRID_Y_MAX) return std::printf("3-D %d %d %d\n", across, ny, r), 1;
+        }
+    // past every height: still within [lo, hi] (the launch then fails with an error)
+    if (pick_rows(1, 2000000, 740, 2, 16, 0.0) != 16) return std::printf("past\n"), 1;
+    for (int tma = 0; tma < 2; ++tma) {
+        if (!tile_fits(2LL * 196605, 196605, tma) || tile_fits(2LL * 196606, 196606, tma)) return std::printf("tall\n"), 1;
+        const int n = tma ? 400000 : 800000;
+        if (!tile_fits(n, 1000, tma) || tile_fits(n + 1, 1000, tma)) return std::printf("cells\n"), 1;
+    }
+    return 0;
+}
+"""
+
+
+def test_launch_extents_hold_for_every_height(tmp_path):
+    src, exe = tmp_path / "plan.cpp", tmp_path / "plan"
+    src.write_text(SOURCE)
+    subprocess.run(["g++", "-std=c++17", "-O2", "-I", os.path.join(ROOT, "dev_field_efvm_b200", "csrc"), str(src),
+                    "-o", str(exe)], check=True)
+    run = subprocess.run([str(exe)], capture_output=True, text=True)
+    assert run.returncode == 0, run.stdout
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("ny", [196605, 196606, 200000])
+@pytest.mark.parametrize("viscous", [0, 1])
+def test_tall_grids_step(ny, viscous):
+    """nx = 2, on both sides of the line: whole steps equal the strip form's at explicit
+    rows (bit for bit without viscous terms, 2e-13 of each variable's scale with)."""
+    import numpy as np
+
+    from dev_field_efvm_b200 import abi, cases
+    from dev_field_efvm_b200.device import Context
+
+    bcs = {s: abi.BC_PERIODIC for s in (abi.XLO, abi.XHI, abi.YLO, abi.YHI)}
+    grid = abi.make_grid(2, ny, hi=(2.0, float(ny), 1.0), bcs=bcs | {abi.ZLO: abi.BC_SLIP_WALL, abi.ZHI: abi.BC_SLIP_WALL})
+    params = abi.make_params(cfl=0.3, r_gas=1.0, reconstruction=abi.RECON_MUSCL, viscous=viscous, mu=1e-3,
+                             viscosity_model=abi.VISC_CONSTANT)
+    rng = np.random.default_rng(ny)
+    f = rng.uniform(-1.0, 1.0, (4, ny, 2))
+    u = cases.prim_to_cons(1.0 + 0.1 * f[0], 0.2 * f[1], 0.2 * f[2], 1.0 + 0.1 * f[3])
+    out = []
+    for form, rows in ((abi.STAGE_AUTO, 0), (abi.STAGE_STRIP, 16)):
+        c = Context(grid, params)
+        c.set_stage_tiling(form, rows)
+        c.upload(u)
+        c.step(1)
+        c.step(2)
+        out.append(c.download())
+        c.close()
+    err = np.max(np.abs(out[0] - out[1]) / np.array([1.0, 1.0, 1.0, 1.0, 3.0]))
+    assert err < 2e-13 if viscous else np.array_equal(out[0], out[1])
+    assert not np.array_equal(out[0], u)
