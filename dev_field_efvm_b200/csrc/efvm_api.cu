@@ -694,6 +694,7 @@ int capture_step_graph(efvm_ctx* c) {
     cudaGraph_t graph;
     CUDA_TRY(c, cudaStreamBeginCapture(S(c), cudaStreamCaptureModeThreadLocal));
     const int rc_enq = enqueue_rk3_step(c);
+    const cudaError_t refused = cudaGetLastError();  // a launch that failed is missing from the graph
     cudaError_t e = cudaStreamEndCapture(S(c), &graph);
     c->graph_kernels = (int)(c->launches - before);
     c->launches = before;
@@ -702,6 +703,10 @@ int capture_step_graph(efvm_ctx* c) {
         return rc_enq;
     }
     if (e != cudaSuccess) return fail(c, EFVM_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
+    if (refused != cudaSuccess) {
+        cudaGraphDestroy(graph);
+        return fail(c, EFVM_ERR_CUDA, std::string("a launch of the step: ") + cudaGetErrorString(refused));
+    }
     e = cudaGraphInstantiate(&c->graph_exec, graph, 0);
     cudaGraphDestroy(graph);
     if (e != cudaSuccess) return fail(c, EFVM_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
@@ -1942,6 +1947,7 @@ int efvm_autotune_stage(efvm_ctx* c, int32_t n_steps, double* best_ms_per_step) 
         if (form == EFVM_STAGE_AUTO) rows.assign(1, 0);
         for (int r : rows) {
             if (r > c->g.ny && r != rows.front()) continue;
+            if (r > 0 && (c->g.ny + r - 1) / r > GRID_Y_MAX) continue;  // no such launch
             c->stage_form = form;
             c->stage_rows = r;
             c->stage_blocks = blocks;
