@@ -490,12 +490,20 @@ int build_ibm_lists3(efvm_ctx* c) {
 
 // Whether the built-in choice is the face-parallel kernel (efvm_tile.cu): an FP64
 // case without explicit form, rows and blocks, within the limits of tile_fits.
+//
+// Any split into slabs gives the unsplit result bit for bit, so a slab's kernel may
+// differ from the unsplit grid's only where the two have the same bits: the plain
+// inviscid forms round every operation explicitly.  With viscous terms (whose
+// reciprocals are formed differently), a body force or a sponge, a slab counts the
+// cells and rows of the whole grid.
 bool use_tile(const efvm_ctx* c) {
     if (c->g.nz > 1 || c->ph.precision != EFVM_PREC_FP64 || c->stage_form != EFVM_STAGE_AUTO || c->stage_rows != 0 ||
         c->stage_blocks != 0)
         return false;
     const bool tma = c->tmaps && stage_tma_eligible(c->g, c->ph, c->ibm, c->nn != nullptr);
-    return tile_fits((long long)c->g.nx * c->g.ny, c->g.ny, tma);
+    const bool same_bits = !c->ph.viscous && !c->ph.sponge && c->ph.body_force_x == 0.0;
+    const int ny = same_bits ? c->g.ny : c->grid.ny;
+    return tile_fits((long long)c->g.nx * ny, ny, tma);
 }
 
 // With corrections the face-parallel stages leave the network's inputs of their
