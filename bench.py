@@ -494,8 +494,8 @@ def tune(ctx, d3):
     if d3:
         return None
     ms = ctx.autotune_stage(5)
-    form, rows, blocks = ctx.stage_tiling()
-    return {"form": "tma" if form == abi.STAGE_TMA else "strip", "rows_per_warp": rows,
+    kernel, rows, blocks = ctx.stage_kernel()
+    return {"form": {abi.KERNEL_TMA: "tma", abi.KERNEL_FACES: "faces"}.get(kernel, "strip"), "rows_per_warp": rows,
             "blocks_per_sm": blocks, "tuner_ms_per_step": ms}
 
 
@@ -746,6 +746,8 @@ def main():
                 "kernel": ("stage3_kernel (fused 3-D MUSCL/HLLC/RK3 substage, x/y/z faces)" if d3
                            else "stage_tma_kernel (fused MUSCL/HLLC/RK3 substage, rows fed by TMA into a "
                                 "shared-memory ring)" if tiling and tiling.get("form") == "tma"
+                           else "tile_stage_kernel (fused MUSCL/HLLC/RK3 substage, one face per lane)"
+                           if tiling and tiling.get("form") == "faces"
                            else "stage_kernel (fused MUSCL/HLLC/RK3 substage)"),
                 "bytes_per_cell_update": bytes_per_cell_update, "cells_per_launch": cells,
                 "stage_ms_per_launch": stage_ms_per_launch,

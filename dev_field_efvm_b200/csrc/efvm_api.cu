@@ -488,22 +488,32 @@ int build_ibm_lists3(efvm_ctx* c) {
     return EFVM_OK;
 }
 
-// Whether the built-in choice is the face-parallel kernel (efvm_tile.cu): an FP64
-// case without explicit form, rows and blocks, within the limits of tile_fits.
+// Whether the face-parallel kernel (efvm_tile.cu) may run the case: FP64, 2-D, within
+// the limits of tile_fits.
 //
 // Any split into slabs gives the unsplit result bit for bit, so a slab's kernel may
 // differ from the unsplit grid's only where the two have the same bits: the plain
 // inviscid forms round every operation explicitly.  With viscous terms (whose
 // reciprocals are formed differently), a body force or a sponge, a slab counts the
 // cells and rows of the whole grid.
-bool use_tile(const efvm_ctx* c) {
-    if (c->g.nz > 1 || c->ph.precision != EFVM_PREC_FP64 || c->stage_form != EFVM_STAGE_AUTO || c->stage_rows != 0 ||
-        c->stage_blocks != 0)
-        return false;
+bool tile_applies(const efvm_ctx* c) {
+    if (c->g.nz > 1 || c->ph.precision != EFVM_PREC_FP64) return false;
     const bool tma = c->tmaps && stage_tma_eligible(c->g, c->ph, c->ibm, c->nn != nullptr);
     const bool same_bits = !c->ph.viscous && !c->ph.sponge && c->ph.body_force_x == 0.0;
     const int ny = same_bits ? c->g.ny : c->grid.ny;
     return tile_fits((long long)c->g.nx * ny, ny, tma);
+}
+
+// The setting that efvm_get_stage_tiling reports for it: the strip form, one row per
+// warp and the strip form's built-in block count, both explicit.
+bool names_tile(const efvm_ctx* c, int form, int rows, int blocks) {
+    return form == EFVM_STAGE_STRIP && rows == 1 && blocks == stage_blocks_per_sm(false, c->ph.viscous != 0, false);
+}
+
+// Whether a stage runs it: the built-in choice where it applies.
+bool use_tile(const efvm_ctx* c) {
+    const bool built_in = c->stage_form == EFVM_STAGE_AUTO && c->stage_rows == 0 && c->stage_blocks == 0;
+    return (built_in || names_tile(c, c->stage_form, c->stage_rows, c->stage_blocks)) && tile_applies(c);
 }
 
 // With corrections the face-parallel stages leave the network's inputs of their
@@ -1868,10 +1878,10 @@ static int resolved_blocks(const efvm_ctx* c, int form) {
 
 int efvm_get_stage_tiling(efvm_ctx* c, int32_t* form, int32_t* rows_per_warp, int32_t* blocks_per_sm) {
     if (!c || !form || !rows_per_warp || !blocks_per_sm) return fail(c, EFVM_ERR_INVALID_ARG, "null argument");
-    if (use_tile(c)) {  // the face-parallel build counts as the strip form's
+    if (use_tile(c)) {  // the setting that names the face-parallel kernel
         *form = EFVM_STAGE_STRIP;
-        *rows_per_warp = TILE_ROWS;
-        *blocks_per_sm = resolved_blocks(c, EFVM_STAGE_STRIP);
+        *rows_per_warp = 1;
+        *blocks_per_sm = stage_blocks_per_sm(false, c->ph.viscous != 0, false);
         return EFVM_OK;
     }
     *form = resolved_form(c);
@@ -1884,6 +1894,28 @@ int efvm_get_stage_tiling(efvm_ctx* c, int32_t* form, int32_t* rows_per_warp, in
         // the built-in rows follow the resident slots of the count in use
         *rows_per_warp = stage_rows_for(c->g.nx, c->g.ny, *blocks_per_sm);
     }
+    if (names_tile(c, *form, *rows_per_warp, *blocks_per_sm) && tile_applies(c)) *blocks_per_sm = 0;  // the strip kernel
+    return EFVM_OK;
+}
+
+int efvm_get_stage_kernel(efvm_ctx* c, int32_t* kernel, int32_t* rows, int32_t* blocks_per_sm) {
+    if (!c || !kernel || !rows || !blocks_per_sm) return fail(c, EFVM_ERR_INVALID_ARG, "null argument");
+    if (use_tile(c)) {
+        *kernel = EFVM_KERNEL_FACES;
+        *rows = TILE_ROWS;
+        *blocks_per_sm = TILE_BLOCKS;
+        return EFVM_OK;
+    }
+    if (is_3d(c)) {
+        *kernel = EFVM_KERNEL_STRIP;
+        stage3_tiling(c->g, c->ph, rows, blocks_per_sm);
+        return EFVM_OK;
+    }
+    int32_t form;
+    const int rc = efvm_get_stage_tiling(c, &form, rows, blocks_per_sm);
+    if (rc) return rc;
+    *kernel = form == EFVM_STAGE_TMA ? EFVM_KERNEL_TMA : EFVM_KERNEL_STRIP;
+    *blocks_per_sm = resolved_blocks(c, form);
     return EFVM_OK;
 }
 

@@ -280,6 +280,8 @@ int batch_form_blocks(bool fp32, bool viscous);
 int stage_strips(int nx);
 int stage_rows(int nx, int ny, bool fp32, bool viscous, bool tma = false);
 int stage_rows_for(int nx, int ny, int blocks_per_sm);
+// The same of the 3-D stage kernel.
+void stage3_tiling(const Geometry& g, const Physics& ph, int32_t* rows, int32_t* blocks_per_sm);
 // Resident blocks per SM of the stage-kernel form (tma: the TMA-fed kernel), and
 // the strip form's second choice for the autotuner (0: none).
 int stage_blocks_per_sm(bool fp32, bool viscous, bool tma);

@@ -1498,6 +1498,10 @@ int stage_rows(int nx, int ny, bool fp32, bool viscous, bool tma) {
     return rows_per_warp(nx, ny, tma ? tma_resident(fp32) : form_minb(fp32, viscous));
 }
 int stage_rows_for(int nx, int ny, int blocks_per_sm) { return rows_per_warp(nx, ny, blocks_per_sm); }
+void stage3_tiling(const Geometry& g, const Physics& ph, int32_t* rows, int32_t* blocks_per_sm) {
+    *rows = rows_per_warp3(g, strip_width3(g.nx, ph.viscous != 0));
+    *blocks_per_sm = MINB3;
+}
 int stage_blocks_per_sm(bool fp32, bool viscous, bool tma) { return tma ? tma_resident(fp32) : form_minb(fp32, viscous); }
 
 int stage_alt_blocks(bool fp32, bool viscous) {

@@ -888,11 +888,19 @@ __global__ void __launch_bounds__(IBM_THREADS) ibm3_kernel(Geometry g, Physics p
 // mesh, else 31.
 static int strip_width3(int nx, bool visc) { return !visc && (nx + 31) / 32 < (nx + 30) / 31 ? 32 : 31; }
 
+// Blocks side by side (strips x groups of layers), and the rows each marches.
+static long long blocks_across3(const Geometry& g, int width) {
+    return (long long)((g.nx + width - 1) / width) * ((g.nz + WPB3 - 1) / WPB3);
+}
+static int rows_per_warp3(const Geometry& g, int width) {
+    return pick_rows(blocks_across3(g, width), g.ny, 148LL * MINB3, 2, ROWS3, 0.15);
+}
+
 template <int SCHEME, int RECON, bool VISC, int LIM, bool PXYZ>
 static void launch_stage3_k(const StageArgs& a, bool pdl, cudaStream_t s) {
     const int width = strip_width3(a.g.nx, VISC);
-    const long long across = (long long)((a.g.nx + width - 1) / width) * ((a.g.nz + WPB3 - 1) / WPB3);
-    const int rows = pick_rows(across, a.g.ny, 148LL * MINB3, 2, ROWS3, 0.15);
+    const long long across = blocks_across3(a.g, width);
+    const int rows = rows_per_warp3(a.g, width);
     dim3 grid((unsigned)across, (a.g.ny + rows - 1) / rows);
     launch_k(stage3_kernel<SCHEME, RECON, VISC, LIM, PXYZ>, grid, dim3(32 * WPB3), s, pdl, a, rows, width);
 }

@@ -33,9 +33,10 @@ def main() -> None:
         c.set_stage_tiling(FORMS[args.form], args.rows)
         c.upload(u)
         c.step(args.steps)
-        form, rows, _ = c.stage_tiling()
+        kernel, rows, _ = c.stage_kernel()
+        name = {abi.KERNEL_TMA: "tma", abi.KERNEL_FACES: "faces"}.get(kernel, "strip")
         print(f"{args.steps} steps of the {args.n}^2 vortex, {args.precision}, "
-              f"form {'tma' if form == abi.STAGE_TMA else 'strip'}, {rows} rows per warp: "
+              f"kernel {name}, {rows} rows: "
               f"step {c.solver_state().step}")
 
 

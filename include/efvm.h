@@ -354,12 +354,14 @@ int efvm_profile_steps(efvm_ctx* ctx, int64_t n_steps, double out_ms[4]);
  * the strip form whatever is set.
  * EFVM_STAGE_AUTO is the built-in choice: the TMA-fed form wherever the case
  * allows it (the faster of the two at 4096^2 in both precisions), else the
- * strip form; an FP64 case of up to 400,000 cells (800,000 where the TMA-fed
- * form does not run) without explicit rows or blocks runs a build of the strip form with one face per lane (reported by
- * efvm_get_stage_tiling as the strip form).  Both give the reference's results
- * (the forms, and the strip form's builds for different block counts, differ
- * from each other by a few ulps at most; a form gives the same bits for any
- * rows per warp). */
+ * strip form.  An FP64 case of up to 400,000 cells (800,000 where the TMA-fed
+ * form does not run) and 196,605 rows without explicit rows or blocks runs the
+ * face-parallel kernel instead, one face per lane; a slab with viscous terms, a
+ * body force or a sponge counts the whole grid's cells and rows.  FP32 fluxes have
+ * no face-parallel kernel, so on such small grids they are the slower choice.
+ * All give the reference's results (the kernels, and the strip form's builds for
+ * different block counts, differ from each other by a few ulps at most; a
+ * kernel gives the same bits for any rows per warp). */
 typedef enum { EFVM_STAGE_AUTO = 0, EFVM_STAGE_STRIP = 1, EFVM_STAGE_TMA = 2 } efvm_stage_form;
 /* Select the form, the rows each warp marches and the strip form's resident
  * blocks per SM (0 = built-in choice for each; the FP64 inviscid strip form is
@@ -368,8 +370,18 @@ typedef enum { EFVM_STAGE_AUTO = 0, EFVM_STAGE_STRIP = 1, EFVM_STAGE_TMA = 2 } e
  * runs its systems on the CPU and has no counterpart; this replaces no call.
  * EFVM_ERR_UNSUPPORTED for EFVM_STAGE_TMA on a 3-D context. */
 int efvm_set_stage_tiling(efvm_ctx* ctx, int32_t form, int32_t rows_per_warp, int32_t blocks_per_sm);
-/* The form the context's next stage runs, its rows per warp and blocks per SM. */
+/* The setting of the context's next stage: form, rows per warp and blocks per SM,
+ * in terms of efvm_set_stage_tiling, so that setting it again changes nothing.
+ * The face-parallel kernel has no form of its own there: EFVM_STAGE_STRIP with 1
+ * row (each of its warps covers one) and the strip form's built-in block count,
+ * both given, names it where the case is within its limits (above); there the strip
+ * kernel itself at 1 row is reported with block count 0. */
 int efvm_get_stage_tiling(efvm_ctx* ctx, int32_t* form, int32_t* rows_per_warp, int32_t* blocks_per_sm);
+/* The kernel the context's next stage runs, the rows of one of its warps (of a
+ * tile for the face-parallel kernel) and the resident blocks per SM it is built
+ * for.  A 3-D context reports its strip kernel.  No counterpart in the reference. */
+typedef enum { EFVM_KERNEL_STRIP = 1, EFVM_KERNEL_TMA = 2, EFVM_KERNEL_FACES = 3 } efvm_stage_kernel;
+int efvm_get_stage_kernel(efvm_ctx* ctx, int32_t* kernel, int32_t* rows, int32_t* blocks_per_sm);
 /* Time n_steps whole steps (default 3) of every candidate tiling on the live
  * state -- each form the case allows (the strip form at each block count it is
  * built for), with 4, 8, 16 and 32 rows per warp and with the rows that put the
