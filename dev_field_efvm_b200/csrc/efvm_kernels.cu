@@ -200,7 +200,6 @@ __device__ __forceinline__ void stage_strip_src(const A& a, int rows, int strip,
         if constexpr (CG) machine((volatile DevState*)a.st);
         else machine(a.st);
     }
-    constexpr bool BATCH = !std::is_same<A, StageArgs>::value;
     const int i0 = strip * STRIP;
     const int jb = by * rows;
     double lam = 0.0;
@@ -396,7 +395,7 @@ __device__ __forceinline__ void stage_strip_src(const A& a, int rows, int strip,
                     side(q0.mx, q1.mx, q2.mx, q3.mx, l.mx, r.mx);
                     side(q0.my, q1.my, q2.my, q3.my, l.my, r.my);
                     side(q0.E, q1.E, q2.E, q3.E, l.E, r.E);
-                    fx = face_flux<SCHEME, R, BATCH>(xq(l), xq(r), rg, rgm1);
+                    fx = face_flux<SCHEME, R>(xq(l), xq(r), rg, rgm1);
                 } else {
                     V4<R> ul = shfl_up_v(row_c(), 1), ur = shfl_down_v(row_c(), 1);
                     V4<R> ull = ul;  // column i-2 (lane 0 only)
@@ -415,9 +414,9 @@ __device__ __forceinline__ void stage_strip_src(const A& a, int rows, int strip,
                             if constexpr (FP64) slope_faces(limiter, ull, ul, row_c(), R(0.5), R(0), lp, unused);
                             else slope_faces_half(limiter, ull, ul, row_c(), lp, unused);
                         }
-                        fx = face_flux<SCHEME, R, BATCH>(xq(rec_l ? lp : ul), xq(rec_r ? mm : row_c()), rg, rgm1);
+                        fx = face_flux<SCHEME, R>(xq(rec_l ? lp : ul), xq(rec_r ? mm : row_c()), rg, rgm1);
                     } else {
-                        fx = face_flux<SCHEME, R, BATCH>(xq(ul), xq(row_c()), rg, rgm1);
+                        fx = face_flux<SCHEME, R>(xq(ul), xq(row_c()), rg, rgm1);
                     }
                 }
                 const Q4<R> fxr = shfl_down_q(fx, 1);  // face on the right of column i
@@ -437,13 +436,13 @@ __device__ __forceinline__ void stage_strip_src(const A& a, int rows, int strip,
                 else slope_faces_half(limiter, row_c(), row_n(), row_n2(), pn, mn);
                 put_pc(pn);
                 if constexpr (Y_FACTORS) {
-                    gt = face_flux<SCHEME, R, BATCH>(yq(pcr), yq(mn), rg, rgm1);
+                    gt = face_flux<SCHEME, R>(yq(pcr), yq(mn), rg, rgm1);
                 } else {
                     const bool rb = rec_below(j), rt = rec_above(j);
-                    gt = face_flux<SCHEME, R, BATCH>(yq(rb ? pcr : row_c()), yq(rt ? mn : row_n()), rg, rgm1);
+                    gt = face_flux<SCHEME, R>(yq(rb ? pcr : row_c()), yq(rt ? mn : row_n()), rg, rgm1);
                 }
             } else {
-                gt = face_flux<SCHEME, R, BATCH>(yq(row_c()), yq(row_n()), rg, rgm1);
+                gt = face_flux<SCHEME, R>(yq(row_c()), yq(row_n()), rg, rgm1);
             }
             if (!XFIRST && row) x_face();
 

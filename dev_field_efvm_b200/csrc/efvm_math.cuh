@@ -41,14 +41,12 @@ __device__ __forceinline__ double rcp_(double b) {
     const double e = fma(-b, r, 1.0);
     return fma(r, fma(e, e, e), r);
 }
-// FP32: the approximate instruction itself.  __fdividef and rsqrtf give the same
-// bits for normal inputs, but wrap it in a denormal check and a rescale (4 % of
-// the FP32-flux step at 4096^2: 1.440 -> 1.383 ms).
-__device__ __forceinline__ float rcp_(float b) {
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
-    return r;
-}
+// FP32: the library functions, which also take subnormal arguments: thin gases reach
+// them (den X in hllc_flux is about 4 rho^3 a^4).  The .ftz instructions give the same
+// bits for normal arguments but infinity below them; they ran 4 % faster (FP32-flux
+// step at 4096^2: 1.380 against 1.437 ms).  Taking them first and repeating a flux
+// that is not finite with these functions was no faster (1.436 to 1.496 ms).
+__device__ __forceinline__ float rcp_(float b) { return __fdividef(1.0f, b); }
 // 1/sqrt(x) from the PTX approximate rsqrt.approx.ftz.f64 seed y0 and one
 // third-order step of the binomial series 1/sqrt(x) = y0 (1 - e)^(-1/2) with
 // e = 1 - x y0^2: y0 + y0 e (1/2 + 3e/8), relative error about 5e^3/16 before
@@ -59,20 +57,9 @@ __device__ __forceinline__ double rsqrt_(double x) {
     const double e = fma(-x * y, y, 1.0);
     return fma(y * e, fma(e, 0.375, 0.5), y);
 }
-__device__ __forceinline__ float rsqrt_(float x) {
-    float r;
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
-// The batch kernels keep rsqrtf: with the instruction the compiler fuses the
-// sound speed's product differently there, which moves their FP32 fluxes by
-// roundings.
-template <bool BATCH>
-__device__ __forceinline__ float rsqrt_of(float x) {
-    return BATCH ? rsqrtf(x) : rsqrt_(x);
-}
-// The smallest normal value: the .ftz seeds above flush anything below it to
-// zero (and return infinity for it), so their callers keep inputs above it.
+__device__ __forceinline__ float rsqrt_(float x) { return rsqrtf(x); }
+// The smallest normal value: the .ftz seeds of the FP64 functions flush anything
+// below it to zero (and return infinity for it).
 template <class R>
 __device__ __forceinline__ R normal_min();
 template <>
@@ -88,7 +75,7 @@ template <class R>
 struct Side {
     R inv, un, ut, q, p, a;
 };
-template <bool BATCH, class R>
+template <class R>
 __device__ __forceinline__ Side<R> side_with(const Q4<R>& u, R inv, R gamma, R gm1) {
     Side<R> s;
     s.inv = inv;
@@ -97,16 +84,16 @@ __device__ __forceinline__ Side<R> side_with(const Q4<R>& u, R inv, R gamma, R g
     s.q = s.un * s.un + s.ut * s.ut;
     s.p = gm1 * (u.E - R(0.5) * u.r * s.q);
     const R a2 = gamma * s.p * s.inv;
-    s.a = a2 * rsqrt_of<BATCH>(a2);  // sqrt(a2); NaN for a non-physical p <= 0, which the stage flags
+    s.a = a2 * rsqrt_(a2);  // sqrt(a2); NaN for a non-physical p <= 0, which the stage flags
     return s;
 }
 // Both sides of a face, with 1/rho_L = rho_R w and 1/rho_R = rho_L w from one
 // reciprocal w = 1/(rho_L rho_R) (a few ulps from the two separate reciprocals).
-template <bool BATCH, class R>
+template <class R>
 __device__ __forceinline__ void sides_of(const Q4<R>& L, const Q4<R>& Rr, R gamma, R gm1, Side<R>& l, Side<R>& r) {
     const R w = rcp_(L.r * Rr.r);
-    l = side_with<BATCH>(L, Rr.r * w, gamma, gm1);
-    r = side_with<BATCH>(Rr, L.r * w, gamma, gm1);
+    l = side_with(L, Rr.r * w, gamma, gm1);
+    r = side_with(Rr, L.r * w, gamma, gm1);
 }
 
 // physical_flux_inline along the face normal for a state with known normal
@@ -243,10 +230,10 @@ __device__ __forceinline__ Q4<double> hllc_flux_d(const Q4<double>& L, const Q4<
 }
 
 // Rusanov::flux_inline, crates/cfd_riemann/src/lib.rs:222-240
-template <bool BATCH, class R>
+template <class R>
 __device__ __forceinline__ Q4<R> rusanov_flux(const Q4<R>& L, const Q4<R>& Rr, R gamma, R gm1) {
     Side<R> l, r;
-    sides_of<BATCH>(L, Rr, gamma, gm1, l, r);
+    sides_of(L, Rr, gamma, gm1, l, r);
     const Q4<R> fl = physical_flux(L.r, l.un, l.ut, L.E, l.p);
     const Q4<R> fr = physical_flux(Rr.r, r.un, r.ut, Rr.E, r.p);
     const R hl = R(0.5) * fmax_(fabs_(l.un) + l.a, fabs_(r.un) + r.a);
@@ -275,10 +262,10 @@ __device__ __forceinline__ Q4<R> rusanov_flux(const Q4<R>& L, const Q4<R>& Rr, R
 //    is formed, s_* and 1/(f_K (s_K - s_*)) = d/(f_K (s_K d - n)) come from one
 //    reciprocal of d f_K (s_K d - n).
 // The results agree with the literal evaluation to a few ulps.
-template <class R, bool THORNBER, bool BATCH>
+template <class R, bool THORNBER>
 __device__ __forceinline__ Q4<R> hllc_flux(const Q4<R>& L, const Q4<R>& Rr, R gamma, R gm1) {
     Side<R> l, r;
-    sides_of<BATCH>(L, Rr, gamma, gm1, l, r);
+    sides_of(L, Rr, gamma, gm1, l, r);
     R lcn = l.un, lct = l.ut, rcn = r.un, rct = r.ut, ELc = L.E, ERc = Rr.E;
     if (THORNBER) {
         const R vmax2 = fmax_(l.q, r.q);
@@ -290,7 +277,7 @@ __device__ __forceinline__ Q4<R> hllc_flux(const Q4<R>& L, const Q4<R>& Rr, R ga
         // any representable change of the flux.
         const R amax2 = amax * amax;
         const R prod = vmax2 * amax2;
-        const R z = (vmax2 >= amax2) ? R(1) : (prod >= normal_min<R>() ? vmax2 * rsqrt_of<BATCH>(prod) : R(0));
+        const R z = (vmax2 >= amax2) ? R(1) : (prod >= normal_min<R>() ? vmax2 * rsqrt_(prod) : R(0));
         const R avgn = R(0.5) * (l.un + r.un), avgt = R(0.5) * (l.ut + r.ut);
         const R hz = R(0.5) * z;
         const R dvn = hz * (l.un - r.un), dvt = hz * (l.ut - r.ut);
@@ -337,14 +324,14 @@ __device__ __forceinline__ Q4<R> hllc_flux(const Q4<R>& L, const Q4<R>& Rr, R ga
     return f;
 }
 
-template <int SCHEME, class R, bool BATCH = false>
+template <int SCHEME, class R>
 __device__ __forceinline__ Q4<R> face_flux(const Q4<R>& L, const Q4<R>& Rr, R gamma, R gm1) {
     if constexpr (sizeof(R) == sizeof(double)) {
         if (SCHEME == EFVM_FLUX_RUSANOV) return rusanov_flux_d(L, Rr, gamma, gm1);
         return hllc_flux_d<SCHEME != EFVM_FLUX_HLLC_TEXTBOOK>(L, Rr, gamma, gm1);
     } else {
-        if (SCHEME == EFVM_FLUX_RUSANOV) return rusanov_flux<BATCH>(L, Rr, gamma, gm1);
-        return hllc_flux<R, SCHEME != EFVM_FLUX_HLLC_TEXTBOOK, BATCH>(L, Rr, gamma, gm1);
+        if (SCHEME == EFVM_FLUX_RUSANOV) return rusanov_flux(L, Rr, gamma, gm1);
+        return hllc_flux<R, SCHEME != EFVM_FLUX_HLLC_TEXTBOOK>(L, Rr, gamma, gm1);
     }
 }
 
