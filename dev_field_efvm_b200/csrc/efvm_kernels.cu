@@ -1306,7 +1306,7 @@ static int form_minb(bool fp32, bool viscous) {
 // TMA-fed form: 8 rows 2.04, 16 rows 1.97, 32 rows 1.98).
 static int rows_per_warp(int nx, int ny, int blocks_per_sm) {
     const long long across = ((nx + STRIP - 1) / STRIP + WPB - 1) / WPB;
-    return pick_rows(across, ny, 148LL * blocks_per_sm, 2, 16, 0.0);
+    return pick_rows(across, ny, 148LL * blocks_per_sm, 2, 16);
 }
 
 template <int SCHEME, int RECON, class R, bool VISC>

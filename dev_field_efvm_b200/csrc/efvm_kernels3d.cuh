@@ -893,7 +893,7 @@ static long long blocks_across3(const Geometry& g, int width) {
     return (long long)((g.nx + width - 1) / width) * ((g.nz + WPB3 - 1) / WPB3);
 }
 static int rows_per_warp3(const Geometry& g, int width) {
-    return pick_rows(blocks_across3(g, width), g.ny, 148LL * MINB3, 2, ROWS3, 0.15);
+    return pick_rows(blocks_across3(g, width), g.ny, 148LL * MINB3, 2, ROWS3);
 }
 
 template <int SCHEME, int RECON, bool VISC, int LIM, bool PXYZ>

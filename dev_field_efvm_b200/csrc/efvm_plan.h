@@ -11,36 +11,47 @@ constexpr int GRID_Y_MAX = 65535;  // blocks along a launch's y
 // Rows of a tile of the face-parallel kernel (efvm_tile.cu).
 constexpr int TILE_ROWS = 3;
 
-// Rows each warp marches: the count in [lo, hi] whose blocks, dealt to the resident
-// slots in order, finish first.  A block of r rows takes r passes, one more that
-// only forms the face below its first row (about half a pass), and the column's
-// last block is shorter.  A count that leaves a few full blocks for one more wave
-// pays for nearly two: by the fewest-rows rule that this one replaces 1024^2 took
-// 12 rows and 1.05 waves (us per step 193 -> 159), 4400x820 viscous 804 -> 742.
-// In 3-D short last blocks fill the gaps the long ones leave (tail_cost 0.15:
-// over nine cases of 50 to 256 cells a side the choice is within 0.9 % of the best
-// of 2..16 rows on average, 3 % at most; without it 1.7 and 6 %); in 2-D the same
-// term made 1024^2 5 % and 4096^2 3 % slower.
+// When the last block of a stage ends, in half passes, if `slots` blocks run at a time
+// and each free slot takes the next one.  A block of r rows takes r passes and one
+// more that only forms the face below its first row (about half a pass); `across`
+// blocks lie side by side, and the last ones of the columns, launched last, are
+// shorter and fill the slots that the full ones leave free.
+inline long long stage_end(long long across, int ny, long long slots, int rows) {
+    const int down = (ny + rows - 1) / rows;
+    const long long full = 2LL * rows + 1, tail = 2LL * (ny - (down - 1) * rows) + 1;
+    const long long blocks = across * (down - 1), begun = blocks / slots * full, over = blocks % slots;
+    auto ceil_div = [](long long x, long long y) { return x > 0 ? (x + y - 1) / y : 0; };
+    if (over == 0) return begun + ceil_div(across, slots) * tail;
+    // `over` slots run one more full block; the others take tails from `begun` on
+    const long long idle = slots - over;
+    if (ceil_div(across, idle) * tail <= full) return begun + full;
+    const long long before = full / tail, past = ceil_div(full, tail);
+    const long long on_idle = std::max(past, ceil_div(across + over * past, slots)) * tail;
+    const long long on_last = full + ceil_div(across - idle * before, slots) * tail;
+    return begun + std::min(on_idle, on_last);
+}
+
+// Rows each warp marches, in [lo, hi]: the fewest whose blocks fit the resident slots
+// at once, unless another count ends the stage at least 8 % earlier by stage_end.
+// The fewest-rows rule alone pays for a whole wave where it is cut off at hi or leaves
+// a few blocks over: 1024^2 took 12 rows and 1.05 waves (us per step 193 -> 159),
+// 4400x820 viscous 804 -> 742.  Over 120 2-D grids of 60,000 to 17 million cells,
+// most of them random, in four forms the choice is 0.6 % from the best of 2..16 rows on average
+// (fewest rows 7.3 %), over 68 3-D grids 0.7 % (6.0 %).  The 8 % keep the fewest rows
+// where the estimate does not separate the counts: by stage_end alone 8 of 204 3-D
+// cases ran 3 to 13 % slower than with the fewest rows, so 4, by up to 5 %.
 //
 // The blocks of a column lie along the launch's y, so a tall grid takes at least
-// the rows that fit its column there (ny = 900,000 at six blocks per SM: by cost
-// alone 13 rows, 69,231 blocks).
-inline int pick_rows(long long across, int ny, long long slots, int lo, int hi, double tail_cost) {
+// the rows that fit its column there.
+inline int pick_rows(long long across, int ny, long long slots, int lo, int hi) {
     lo = std::min(hi, std::max(lo, (ny + GRID_Y_MAX - 1) / GRID_Y_MAX));
-    int best = lo;
-    double best_cost = 1e300;
-    for (int rows = lo; rows <= hi; ++rows) {
-        const int down = (ny + rows - 1) / rows, tail = ny - (down - 1) * rows;
-        const long long blocks = across * down, full = blocks / slots, over = blocks - full * slots;
-        const double last = over == 0 ? 0.0 : (over <= across ? tail + 0.5 : rows + 0.5);
-        const double cost = (double)full * (rows + 0.5) + last + tail_cost * (tail + 0.5);
-        if (cost < best_cost) {
-            best_cost = cost;
-            best = rows;
-        }
-        if (rows >= ny) break;
-    }
-    return best;
+    const int top = std::max(lo, std::min(hi, ny));  // more rows than the grid has change nothing
+    const int fewest = (int)std::min<long long>(top, std::max<long long>(lo, (across * ny + slots - 1) / slots));
+    int best = fewest;
+    for (int rows = lo; rows <= top; ++rows)
+        if (stage_end(across, ny, slots, rows) < stage_end(across, ny, slots, best)) best = rows;
+    const long long end = stage_end(across, ny, slots, best);
+    return 100 * end < 92 * stage_end(across, ny, slots, fewest) ? best : fewest;
 }
 
 // Whether an FP64 case without explicit form, rows and blocks runs the face-parallel
