@@ -501,7 +501,7 @@ bool tile_applies(const efvm_ctx* c) {
     const bool tma = c->tmaps && stage_tma_eligible(c->g, c->ph, c->ibm, c->nn != nullptr);
     const bool same_bits = !c->ph.viscous && !c->ph.sponge && c->ph.body_force_x == 0.0;
     const int ny = same_bits ? c->g.ny : c->grid.ny;
-    return tile_fits((long long)c->g.nx * ny, ny, tma);
+    return tile_fits(c->g.nx, ny, tma);
 }
 
 // The setting that efvm_get_stage_tiling reports for it: the strip form, one row per

@@ -293,8 +293,7 @@ int stage_alt_blocks(bool fp32, bool viscous);
 bool stage_tma_eligible(const Geometry& g, const Physics& ph, bool ibm, bool corr);
 int encode_state_map(const Geometry& g, const double* buf, bool u0, void* map_out);
 // The face-parallel stage kernel (efvm_tile.cu): 2-D FP64 cases, tiles of
-// 31 columns x TILE_ROWS rows, TILE_BLOCKS resident blocks per SM.
-constexpr int TILE_BLOCKS = 4;
+// TILE_COLS columns x TILE_ROWS rows, TILE_BLOCKS resident blocks per SM (efvm_plan.h).
 int launch_stage_tile(const StageArgs& a, bool pdl, void* stream);
 int launch_batch_stage(const BatchStageArgs& b, int n_tiles, bool pdl, void* stream);
 // Per-step set-up of every case (one thread each).

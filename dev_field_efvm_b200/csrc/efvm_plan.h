@@ -55,14 +55,25 @@ inline int pick_rows(long long across, int ny, long long slots, int lo, int hi) 
 }
 
 // Whether an FP64 case without explicit form, rows and blocks runs the face-parallel
-// kernel: up to a number of cells, and where its column of tiles fits the launch.
-// The lines lie where the forms measured equal (us per step, other form /
-// face-parallel): against the TMA-fed form 512^2 57.5 / 53.9, 768^2 95.7 / 106,
-// 1003x777 121 / 140; against the viscous strip form 1500x279 113 / 105, 2200x410
-// 203 / 203.
-constexpr long long TILE_CELLS_TMA = 400000, TILE_CELLS_STRIP = 800000;
-inline bool tile_fits(long long cells, int ny, bool tma_applies) {
-    return cells <= (tma_applies ? TILE_CELLS_TMA : TILE_CELLS_STRIP) && (ny + TILE_ROWS - 1) / TILE_ROWS <= GRID_Y_MAX;
+// kernel, by its grid.  Up to one wave of tiles it always does: there a stage is one
+// tile's latency (10,000 x 1 cells: 14.4 us per step against 20.5).  Above, up to a
+// number of cells, which lies where the forms measured equal: 300,000 against the
+// TMA-fed form (us per step, TMA-fed / face-parallel, 512^2 58 / 54, 600^2 66 / 72,
+// 800 x 500 67 / 76), 815,000 against the viscous strip form (2000 x 400 171 / 162,
+// 2200 x 410 203 / 203).  A tile costs the same however many of its rows the grid
+// fills, and a flat grid leaves the strips' marches short as well, so the line falls
+// with the cube of rows in whole tiles to rows: at ny = 1 the tiles lose from one
+// wave on (60,000 cells 39 us against 28, 400,000 220 against 113), at ny = 4 from
+// about 100,000 cells (400,000: 101 against 73).  Over 306 grids of 5,000 to 800,000
+// cells and 1 to 9750 rows the choice is 0.4 % from the faster form on average.
+constexpr int TILE_COLS = 31, TILE_BLOCKS = 4;  // a tile's columns; resident blocks per SM
+constexpr long long TILE_CELLS_TMA = 300000, TILE_CELLS_STRIP = 815000;
+inline bool tile_fits(int nx, int ny, bool tma_applies) {
+    const int down = (ny + TILE_ROWS - 1) / TILE_ROWS;
+    if (down > GRID_Y_MAX) return false;  // the column of tiles lies along the launch's y
+    if ((long long)((nx + TILE_COLS - 1) / TILE_COLS) * down <= 148LL * TILE_BLOCKS) return true;
+    const double f = (double)down * TILE_ROWS / ny;
+    return (double)nx * ny * f * f * f <= (double)(tma_applies ? TILE_CELLS_TMA : TILE_CELLS_STRIP);
 }
 
 }  // namespace efvm

@@ -298,7 +298,8 @@ __global__ void __launch_bounds__(32 * (2 * R + 1), MINB) tile_stage_kernel(cons
 
 template <int SCHEME, int RECON, bool VISC, bool FULL, bool CORR, int LIM, bool PXY>
 void launch_k(const StageArgs& a, bool pdl, cudaStream_t s) {
-        constexpr int R = TILE_ROWS, MINB = TILE_BLOCKS;
+    static_assert(TILE_COLS == STRIP, "the launch rule counts the kernel's tiles");
+    constexpr int R = TILE_ROWS, MINB = TILE_BLOCKS;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((a.g.nx + STRIP - 1) / STRIP, (a.g.ny + R - 1) / R);
     cfg.blockDim = dim3(32 * (2 * R + 1));

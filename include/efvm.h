@@ -354,8 +354,9 @@ int efvm_profile_steps(efvm_ctx* ctx, int64_t n_steps, double out_ms[4]);
  * the strip form whatever is set.
  * EFVM_STAGE_AUTO is the built-in choice: the TMA-fed form wherever the case
  * allows it (the faster of the two at 4096^2 in both precisions), else the
- * strip form.  An FP64 case of up to 400,000 cells (800,000 where the TMA-fed
- * form does not run) and 196,605 rows without explicit rows or blocks runs the
+ * strip form.  An FP64 case of up to about 300,000 cells (815,000 where the TMA-fed
+ * form does not run; fewer on flat grids, whose rows fill the kernel's tiles of
+ * three in part) and 196,605 rows without explicit rows or blocks runs the
  * face-parallel kernel instead, one face per lane; a slab with viscous terms, a
  * body force or a sponge counts the whole grid's cells and rows.  FP32 fluxes have
  * no face-parallel kernel, so on such small grids they are the slower choice.

@@ -29,7 +29,7 @@ def channel(nx, ny):
 @pytest.mark.parametrize("nx,ny,cuts", [
     (1024, 800, (0, 400, 800)),        # 819,200 cells: two slabs below the line
     (1024, 800, (0, 20, 800)),         # one slab far below it, one just below
-    (1021, 787, (0, 5, 787)),          # 803,527 cells, ragged
+    (1021, 807, (0, 5, 807)),          # 823,947 cells, ragged
     (1024, 600, (0, 301, 600)),        # below the line: unsplit and slabs alike
 ])
 def test_viscous_slabs_equal_the_unsplit_context(nx, ny, cuts):

@@ -12,7 +12,8 @@ pytestmark = pytest.mark.gpu
 
 
 def box(nx, ny):
-    bcs = {s: abi.BC_PERIODIC for s in (abi.XLO, abi.XHI, abi.YLO, abi.YHI)}
+    bcs = {abi.XLO: abi.BC_PERIODIC, abi.XHI: abi.BC_PERIODIC}
+    bcs[abi.YLO] = bcs[abi.YHI] = abi.BC_PERIODIC if ny > 1 else abi.BC_SLIP_WALL
     return abi.make_grid(nx, ny, hi=(1.0, ny / nx, 1.0), bcs=bcs | {abi.ZLO: abi.BC_SLIP_WALL, abi.ZHI: abi.BC_SLIP_WALL})
 
 
@@ -28,8 +29,9 @@ F, S, T = abi.KERNEL_FACES, abi.KERNEL_STRIP, abi.KERNEL_TMA
 
 @pytest.mark.parametrize("nx,ny,kw,kernel", [
     (64, 64, {}, F), (64, 64, VISC, F), (64, 64, dict(precision=abi.PREC_FP32_FLUX), T),
-    (64, 64, dict(precision=abi.PREC_FP32_FLUX, **VISC), S), (800, 500, {}, F), (801, 500, {}, T),
-    (1000, 800, VISC, F), (1001, 800, VISC, S), (2, 196605, {}, F), (2, 196606, {}, T), (2, 196606, VISC, S)])
+    (64, 64, dict(precision=abi.PREC_FP32_FLUX, **VISC), S), (1000, 300, {}, F), (1001, 300, {}, T),
+    (1000, 813, VISC, F), (1000, 816, VISC, S), (2, 140000, {}, F), (2, 160000, {}, T), (4, 196605, VISC, F),
+    (4, 196606, VISC, S), (18352, 1, {}, F), (18353, 1, {}, T), (40000, 1, VISC, S)])
 def test_built_in_choice_and_round_trip(nx, ny, kw, kernel):
     c = context(nx, ny, **kw)
     ran, setting = c.stage_kernel(), c.stage_tiling()

@@ -63,9 +63,11 @@ int main() {
     // past every height: still within [lo, hi] (the launch then fails with an error)
     if (pick_rows(1, 2000000, 740, 2, 16) != 16) return std::printf("past\n"), 1;
     for (int tma = 0; tma < 2; ++tma) {
-        if (!tile_fits(2LL * 196605, 196605, tma) || tile_fits(2LL * 196606, 196606, tma)) return std::printf("tall\n"), 1;
-        const int n = tma ? 400000 : 800000;
-        if (!tile_fits(n, 1000, tma) || tile_fits(n + 1, 1000, tma)) return std::printf("cells\n"), 1;
+        if (!tile_fits(1, 196605, tma) || tile_fits(1, 196606, tma)) return std::printf("tall\n"), 1;
+        const int n = (tma ? 300000 : 815000) / 1200;  // rows in whole tiles
+        if (!tile_fits(n, 1200, tma) || tile_fits(n + 1, 1200, tma)) return std::printf("cells\n"), 1;
+        // one row: up to 592 tiles of 31 columns
+        if (!tile_fits(592 * 31, 1, tma) || tile_fits(tma ? 592 * 31 + 1 : 40000, 1, tma)) return std::printf("flat\n"), 1;
     }
     return 0;
 }
