@@ -697,17 +697,23 @@ int enqueue_rk3_step(efvm_ctx* c) {
     return EFVM_OK;
 }
 
+// The side stream of a step with bodies and its events.
+int ensure_side(efvm_ctx* c) {
+    if (!c->ibm || c->side) return EFVM_OK;
+    CUDA_TRY(c, cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking));
+    for (auto& ev : c->ev_fork) CUDA_TRY(c, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+    CUDA_TRY(c, cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming));
+    CUDA_TRY(c, cudaEventCreateWithFlags(&c->ev_forces, cudaEventDisableTiming));
+    return EFVM_OK;
+}
+
 int capture_step_graph(efvm_ctx* c) {
     if (c->graph_exec) {
         cudaGraphExecDestroy(c->graph_exec);
         c->graph_exec = nullptr;
     }
-    if (c->ibm && !c->side) {
-        CUDA_TRY(c, cudaStreamCreateWithFlags(&c->side, cudaStreamNonBlocking));
-        for (auto& ev : c->ev_fork) CUDA_TRY(c, cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-        CUDA_TRY(c, cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming));
-        CUDA_TRY(c, cudaEventCreateWithFlags(&c->ev_forces, cudaEventDisableTiming));
-    }
+    const int rc_side = ensure_side(c);
+    if (rc_side) return rc_side;
     const uint64_t before = c->launches;
     cudaGraph_t graph;
     CUDA_TRY(c, cudaStreamBeginCapture(S(c), cudaStreamCaptureModeThreadLocal));
@@ -1517,6 +1523,11 @@ int efvm_step(efvm_ctx* c, int64_t n_steps, int32_t stop_at_t, double t_stop, do
         if (rc) return rc;
         sync_control(c, stop_at_t, t_stop, cap);
     }
+    // Bodies that move with every step (a driver that integrates them sets them and asks
+    // for one step) would have a graph built for each: its instantiation and first launch
+    // took 215 us of 740 us for such a pair of calls (two discs, 120x390 cells).  One step
+    // on new geometry is launched directly instead; a further one captures the graph.
+    const bool direct = c->ibm && c->geom_dirty && n_steps == 1;
     rc = prologue(c);  // may rebuild the IBM descriptor (first step after set_cylinders)
     if (rc) return rc;
     c->ibm_desc.history = cap ? c->history : nullptr;
@@ -1527,6 +1538,10 @@ int efvm_step(efvm_ctx* c, int64_t n_steps, int32_t stop_at_t, double t_stop, do
             enqueue_substage(c, 3, in, outb, true);
             c->euler_cur ^= 1;
         }
+    } else if (direct) {
+        rc = ensure_side(c);
+        if (!rc) rc = enqueue_rk3_step(c);
+        if (rc) return rc;
     } else {
         if (!c->graph_valid) {
             rc = capture_step_graph(c);
