@@ -558,11 +558,11 @@ int prologue(efvm_ctx* c) {
     return EFVM_OK;
 }
 
-// The stage-kernel form a context runs.  The TMA-fed kernel runs where it is
-// selected and the case allows it (2-D, inviscid, no bodies, no learned
-// correction); EFVM_STAGE_AUTO selects it in both precisions: at 4096^2 it
-// measured 1.70 against 1.85 ms per step (FP32 fluxes) and 2.26 against 2.47
-// (FP64) for the strip kernel.
+// The stage-kernel form a context runs where the face-parallel kernel does not
+// (use_tile).  The TMA-fed kernel runs where it is selected and the case allows it
+// (2-D, inviscid, no bodies, no learned correction); EFVM_STAGE_AUTO selects it in
+// both precisions: at 4096^2 it measures 1.44 against 1.82 ms per step (FP32 fluxes)
+// and 1.64 against 2.38 (FP64) for the strip kernel.
 int resolved_form(const efvm_ctx* c) {
     const bool want = c->stage_form == EFVM_STAGE_TMA || c->stage_form == EFVM_STAGE_AUTO;
     if (want && c->tmaps && stage_tma_eligible(c->g, c->ph, c->ibm, c->nn != nullptr)) return EFVM_STAGE_TMA;
@@ -614,10 +614,10 @@ void enqueue_stage_kernel(efvm_ctx* c, int stage, double* uin, double* uout, boo
     c->launches += launch_stage(a, pdl, S(c));
 }
 
-// The IBM forces of the step graph's last stage run on the next step's side
-// branch, so that the step ends with its last stage.  Anything that reads the forces, or changes what they read (the state,
-// the bodies, the force history's control), first runs them here if a step
-// left them pending: the kernel does nothing otherwise.
+// The IBM forces of a step's last stage run on the next step's side branch, so that
+// the step ends with its last stage.  Anything that reads the forces, or changes what
+// they read (the state, the bodies, the force history's control), first runs them here
+// if a step left them pending: the kernel does nothing otherwise.
 static int finish_forces(efvm_ctx* c) {
     if (!c->ibm) return EFVM_OK;
     if (is_3d(c)) {
@@ -1525,8 +1525,8 @@ int efvm_step(efvm_ctx* c, int64_t n_steps, int32_t stop_at_t, double t_stop, do
     }
     // Bodies that move with every step (a driver that integrates them sets them and asks
     // for one step) would have a graph built for each: its instantiation and first launch
-    // took 215 us of 740 us for such a pair of calls (two discs, 120x390 cells).  One step
-    // on new geometry is launched directly instead; a further one captures the graph.
+    // made such a pair of calls take 694 us where it takes 308 without (two discs, 120x390
+    // cells).  One step on new geometry is launched directly; a further one captures the graph.
     const bool direct = c->ibm && c->geom_dirty && n_steps == 1;
     rc = prologue(c);  // may rebuild the IBM descriptor (first step after set_cylinders)
     if (rc) return rc;

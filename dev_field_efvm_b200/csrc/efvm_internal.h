@@ -206,7 +206,7 @@ struct StageArgs {
     const float* corr;                // learned face-flux corrections [2][4][ny][nx] or null
     float4* prims;                    // face-parallel kernel with corrections: the network's inputs of the
     float prim_gamma;                 // output, [ny][nx] (rho - 1, u, v, p - 1), with the network's gamma
-    int defer_forces;                 // stage 2 of the step graph: its IBM forces run in the next launch
+    int defer_forces;                 // stage 3 of a step: its IBM forces run on the next step's side branch
     // The TMA-fed stage kernel (2-D, inviscid, no bodies, no correction): host
     // copies of the tensor maps (CUtensorMap, 128 bytes) of the stage input and
     // of U^n, copied into the launch's parameters; null selects the strip kernel.

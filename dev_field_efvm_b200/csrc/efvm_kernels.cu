@@ -250,7 +250,6 @@ __device__ __forceinline__ void stage_strip_src(const A& a, int rows, int strip,
             rec_r = ph.periodic_x && true_seam;
         }
         // the same as slope factors (the high words of 0.5 and 0; FP64 TMA-fed form)
-        const bool x_edge = i < NG || i >= g.nx - NG;
         const int fxl = rec_l ? 0x3fe00000 : 0, fxr_ = rec_r ? 0x3fe00000 : 0;
         const bool y_periodic = ph.periodic_y || ph.seam_ylo || ph.seam_yhi;
         const bool seam_rec = y_periodic && true_seam;  // the side across the periodic seam
@@ -1007,10 +1006,12 @@ __device__ __forceinline__ void forces_block(const Geometry& g, const Physics& p
             const double face_area[3] = {dy * dz, dx * dz, dx * dy};
             const double* zf = ib.zfill + ((long long)stage % 3) * ib.n_ghost * 4 + 4LL * k;
             // the step's saved z-ghost state.  Stage 3's forces run after its stage
-            // kernel has counted the step, and the step counter is stable while they
-            // run (the next step's first launch, or the substep call).  The forces of
-            // stages 1 and 2 may run on a side branch while the next stage kernel
-            // counts the step, so they take the parity that the step's set-up recorded.
+            // kernel has counted the step: in a substep call, when they are read, or on
+            // the next step's side branch, which that step's last stage waits for
+            // (ev_forces) before it counts again, so the step counter is stable while
+            // they run.  The forces of stages 1 and 2 may run on the side branch while
+            // the last stage counts the step, so they take the parity that the step's
+            // set-up recorded.
             const int par = stage == 2 ? (int)((st->step - 1ull) & 1ull) : st->step_par;
             const double* z0 = ib.zg0 + 4LL * ((long long)par * ib.n_ghost + k);
             // all neighbour states first (in bounds: the ring of boundary ghosts)
@@ -1323,8 +1324,8 @@ static void launch_stage_t(const StageArgs& a, bool pdl, cudaStream_t s) {
             return;
         }
     }
-    // the viscous MUSCL forms (the strip kernel is the only form of their cases)
-    // are built per limiter, as the TMA-fed form is
+    // the viscous MUSCL forms (FP32 fluxes, and FP64 above the face-parallel kernel's
+    // sizes) are built per limiter, as the TMA-fed form is
     if constexpr (VISC && RECON == EFVM_RECON_MUSCL) {
         if (a.ph.limiter == EFVM_LIMITER_MC)
             launch_k(stage_kernel<SCHEME, RECON, R, F::MINB, VISC, false, F::XFIRST, EFVM_LIMITER_MC>, grid, block, s,

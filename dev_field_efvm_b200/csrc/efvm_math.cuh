@@ -60,7 +60,6 @@ __device__ __forceinline__ double rsqrt_(double x) {
 __device__ __forceinline__ float rsqrt_(float x) { return rsqrtf(x); }
 // 1/sqrt(x) of a normal x >= normal_min: the instruction (the guarded product of
 // hllc_flux; 440x82 cylinder with FP32 fluxes 45.2 -> 44.0 us per step).
-__device__ __forceinline__ double rsqrt_normal(double x) { return rsqrt_(x); }
 __device__ __forceinline__ float rsqrt_normal(float x) {
     float r;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));

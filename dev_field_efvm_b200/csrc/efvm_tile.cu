@@ -19,8 +19,8 @@
 // no shuffles, no halo lanes and no carry to store, and the x and y faces share
 // one copy of the flux code; the price is (R + 1) / R y faces per row and a memory
 // latency and a barrier per tile, which lose to the TMA-fed form where the grid
-// is many waves of tiles.  us per step, strip or TMA form -> this kernel:
-// vortex 64^2 22.6 -> 12.3, 128^2 24.4 -> 14.4, 512^2 57.5 -> 53.9, 768^2 95.7 -> 106;
+// is many waves of tiles (the rule: efvm_plan.h).  us per step, strip or TMA form -> this kernel:
+// vortex 64^2 22.6 -> 12.3, 128^2 24.4 -> 14.4, 512^2 57.7 -> 53.7, 768^2 95.7 -> 106;
 // cylinder 440x82 first order 42.5 -> 26.7, 1100x205 MUSCL 77.7 -> 68.5, 2200x410
 // 203 -> 203.  (Persistent blocks with double-buffered TMA tiles measured 18.5 us at
 // 128^2, 69.5 at 1100x205 and 129 at 1003x777, and won only on large viscous grids,
