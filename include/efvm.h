@@ -85,7 +85,9 @@ typedef enum { EFVM_LIMITER_MINMOD = 0, EFVM_LIMITER_MC = 1 } efvm_limiter;
 typedef enum { EFVM_INTEGRATOR_RK3 = 0, EFVM_INTEGRATOR_EULER = 1 } efvm_integrator;
 typedef enum { EFVM_VISC_SUTHERLAND = 0, EFVM_VISC_CONSTANT = 1 } efvm_viscosity;
 /* FP64: everything in double.  FP32_FLUX: reconstruction and face fluxes in
- * float, stage accumulation, RK combination and marker integral in double. */
+ * float, stage accumulation, RK combination and marker integral in double.  A
+ * face's FP32 intermediates have to stay finite: an HLLC face takes a reciprocal of
+ * about 4 rho^3 a^4, which must be at least 2.9e-39 (rho above 7e-14 at a = 1.2). */
 typedef enum { EFVM_PREC_FP64 = 0, EFVM_PREC_FP32_FLUX = 1 } efvm_precision;
 /* How MUSCL treats the periodic seam.  REFERENCE: the halo-ghost side of a seam
  * face is not reconstructed and has zero slope (crates/cfd_solver/src/lib.rs:
@@ -358,7 +360,8 @@ int efvm_profile_steps(efvm_ctx* ctx, int64_t n_steps, double out_ms[4]);
  * three in part) and 196,605 rows without explicit rows or blocks runs the
  * face-parallel kernel instead, one face per lane; a slab with viscous terms, a
  * body force or a sponge counts the whole grid's cells and rows.  FP32 fluxes have
- * no face-parallel kernel, so on such small grids they are the slower choice.
+ * no face-parallel kernel: up to about 150,000 cells (250,000 with viscous terms)
+ * they are the slower choice.
  * All give the reference's results (the kernels, and the strip form's builds for
  * different block counts, differ from each other by a few ulps at most; a
  * kernel gives the same bits for any rows per warp). */
